@@ -24,8 +24,8 @@
 // gradient), so loads, MMAs and stores of consecutive tiles overlap. Every
 // mbarrier wait is bounded and sets an error flag when it gives up. The
 // backward data pass is the same kernel with the weights transposed and
-// flipped. Weight gradients are a register-tiled FP32 reduction on the CUDA
-// cores.
+// flipped. Weight gradients are a second tensor-core kernel that contracts over
+// the pixels (wgrad_tc_kernel).
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -421,75 +421,262 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
   }
 }
 
-// Weight gradients on the CUDA cores: dW[co][tap][ci] += sum_p G[p][co] X[p + tap][ci],
-// db[co] += sum_p G[p][co]. Thread (cq, ci) owns 4 output channels x 9 taps of one
-// input channel (36 accumulators): per pixel 9 + 4 shared-memory reads for 36 FMAs.
+// Weight gradients on the tensor cores: dW[co][tap][ci] += sum_p G[p][co] X[p + tap][ci],
+// db[co] += sum_p G[p][co]. A contraction over pixels, so both operands are MN-major (a
+// pixel's channels are contiguous). One tile is two output rows y, y + 1 of a 128-pixel
+// column strip: the A operand is the four input rows y - 1 .. y + 2 (M = 128: row r, input
+// channel ci), the B operand the two gradient rows (N = 2 COUT: row g, output channel), and
+// for each horizontal tap dx the same buffer seen 16 dx bytes further on, so 3 x 8 MMAs
+// (K = 16 pixels) give every D_dx[(r, ci)][(g, co)]; the combinations with 0 <= r - g <= 2
+// are dW at dy = r - g, six of eight. Shared memory holds one plane of 16-byte pixel chunks
+// per 8 channels (the no-swizzle layout: planes along M / N, groups of 8 pixels along K),
+// filled by 16-byte asynchronous copies with zeros outside the image; planes are 2080 bytes
+// apart, so the four lanes that copy one pixel write different banks.
+//
+// Warps 0-7 copy the tiles through a four-stage ring, add up their own gradient chunks for
+// db, and every kWgGroup tiles add the finished accumulator (one of two in TMEM) to FP32
+// registers with rounding to nearest, so that the tensor core's own accumulation, which
+// truncates, runs over 32 steps at most (left to run over a CTA's whole share it shrinks the
+// gradients by 1.1e-5; over four tiles by 4e-7); warp 8 issues the MMAs. A warp reads its
+// TMEM lane quarter (row r for 32 input channels) for one gradient row. Barriers are waited
+// on and arrived at by one lane per warp. Every wait is bounded.
+//
+// The CUDA-core kernel this replaced (36 FP32 accumulators per thread, 13 shared-memory
+// reads per 36 FMAs) took 1.40 ms per 32 -> 32 layer of 8 x 512 x 512, 11.0 of the 12.6 ms
+// of a training step; this one 0.147 ms (step 2.73 ms). Its MMAs would take 0.04 ms; the
+// copies bound it: a pixel's 8-channel groups lie in different planes, so data arrive in
+// shared memory 16 bytes at a time (with a quarter of the input rows copied it takes 0.115;
+// fewer MMAs, flushes or bias sums change nothing).
+constexpr int kWgStages = 4;
+constexpr int kWgGroup = 4;                          // tiles accumulated in TMEM before a flush
+constexpr int kWgPlane = kHalo * 16;                 // bytes between planes (2080: 32 mod 128)
+constexpr int kWgXPlanes = 16, kWgGPlanes = 8;       // M = 128, N <= 64
+constexpr int kWgStage = (kWgXPlanes + kWgGPlanes) * kWgPlane;
+constexpr int kWgProducers = 256;                    // warps 0-7
+constexpr int kWgThreads = kWgProducers + 32;
+constexpr int kWgLag = 2;                            // tiles a copy is given to land
+constexpr int kWgTmemCols = 512;
+constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256;
+
+// 16-byte asynchronous copy to shared memory; zeros if !valid (src is not read then).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__((COUT / 4) * CIN) wgrad_kernel(const uint16_t* __restrict__ X,
-                                                                 const uint16_t* __restrict__ Gr, int B, int H,
-                                                                 int W, float* __restrict__ dW,
-                                                                 float* __restrict__ db) {
-  constexpr int NT = (COUT / 4) * CIN;
-  extern __shared__ float wg_smem[];
-  float (*xs)[kHalo][CIN] = reinterpret_cast<float (*)[kHalo][CIN]>(wg_smem);          // [3][kHalo][CIN]
-  float (*gs)[COUT] = reinterpret_cast<float (*)[COUT]>(wg_smem + 3 * kHalo * CIN);    // [kTileM][COUT]
-  const int tid = threadIdx.x;
-  const int ci = tid % CIN, cq = tid / CIN;
-  float acc[4][9];
-  float bacc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 9; ++j) acc[i][j] = 0.0f;
-  const int nseg = (W + kTileM - 1) / kTileM;
-  const long long tiles = (long long)B * H * nseg;
-  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int seg = (int)(t % nseg);
-    const long long by = t / nseg;
-    const int y = (int)(by % H), b = (int)(by / H);
-    const int x0 = seg * kTileM;
-    __syncthreads();
-    for (int i = tid; i < 3 * kHalo * (CIN / 2); i += NT) {
-      const int r = i / (kHalo * (CIN / 2)), rem = i - r * (kHalo * (CIN / 2));
-      const int pix = rem / (CIN / 2), c2 = rem - pix * (CIN / 2);
-      const int yy = y + r - 1, xx = x0 + pix - 1;
-      uint32_t w = 0u;
-      if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-        w = __ldg(reinterpret_cast<const uint32_t*>(X + (((size_t)b * H + yy) * W + xx) * CIN) + c2);
-      xs[r][pix][2 * c2] = bf_lo(w);
-      xs[r][pix][2 * c2 + 1] = bf_hi(w);
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t* __restrict__ X,
+                                                                 const uint16_t* __restrict__ Gr, int B, int H, int W,
+                                                                 float* __restrict__ dW, float* __restrict__ db,
+                                                                 int* __restrict__ err) {
+  constexpr int XC = CIN / 8, GC = COUT / 8;        // 16-byte chunks per pixel
+  constexpr int kN = 2 * COUT;
+  // BF16 x BF16 -> F32, both operands MN-major (bits 15 and 16), M = 128, N = kN
+  constexpr uint32_t kIdesc = idesc_bf16(kN) | (1u << 15) | (1u << 16);
+  extern __shared__ __align__(128) uint8_t wg_smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(wg_smem + kWgStages * kWgStage);
+  uint64_t* empty = full + kWgStages;
+  uint64_t* tfull = empty + kWgStages;   // [2] accumulator complete
+  uint64_t* tempty = tfull + 2;          // [2] accumulator read out
+  uint64_t* mdone = tempty + 2;          // the MMA issuer's last commit
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // planes no copy fills (16 input channels) are read as rows of D that nobody uses
+  for (int i = tid; i < kWgStages * kWgStage / 16; i += kWgThreads)
+    reinterpret_cast<uint4*>(wg_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (tid == 0) {
+    for (int s = 0; s < kWgStages; ++s) {
+      mbar_init(&full[s], kWgProducers / 32);
+      mbar_init(&empty[s], 1);
     }
-    for (int i = tid; i < kTileM * (COUT / 2); i += NT) {
-      const int p = i / (COUT / 2), c2 = i - p * (COUT / 2);
-      const int xx = x0 + p;
-      uint32_t w = 0u;
-      if (xx < W) w = __ldg(reinterpret_cast<const uint32_t*>(Gr + (((size_t)b * H + y) * W + xx) * COUT) + c2);
-      gs[p][2 * c2] = bf_lo(w);
-      gs[p][2 * c2 + 1] = bf_hi(w);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&tfull[s], 1);
+      mbar_init(&tempty[s], kWgProducers / 32);
     }
-    __syncthreads();
-    for (int p = 0; p < kTileM; ++p) {
-      float g[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) g[i] = gs[p][4 * cq + i];
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap) {
-        const float xv = xs[tap / 3][p + tap % 3][ci];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][tap] = fmaf(g[i], xv, acc[i][tap]);
-      }
-      if (ci == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) bacc[i] += g[i];
-      }
-    }
+    mbar_init(mdone, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(kWgTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t smem0 = smem_u32(wg_smem);
+
+  const int nseg = (W + kTileM - 1) / kTileM, npair = (H + 1) / 2;
+  const long long tiles = (long long)B * npair * nseg;
+  const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // this CTA's tiles (grid <= tiles)
+
+  if (warp < 8) {
+    // ---- copies, bias sums and flushes ---------------------------------------------------------
+    const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter and gradient row this warp flushes
+    const int m = q * 32 + lane;            // row of D
+    const int r = m / CIN, ci = m - r * CIN, dy = r - g;
+    // copies: this thread's 8-channel group and first pixel of the input and the gradient rows
+    constexpr int kXStep = kWgProducers / XC, kGStep = kWgProducers / GC;
+    static_assert(kTileM % kXStep == 0 && kTileM % kGStep == 0, "whole passes over a row");
+    const int xc = tid % XC, xp = tid / XC, gc = tid % GC, gp = tid / GC;
+    float acc[3][COUT];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int co = 4 * cq + i;
+    for (int dx = 0; dx < 3; ++dx)
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) atomicAdd(dW + ((size_t)co * 9 + tap) * CIN + ci, acc[i][tap]);
-    if (ci == 0) atomicAdd(db + co, bacc[i]);
+      for (int c = 0; c < COUT; ++c) acc[dx][c] = 0.0f;
+    float bacc[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) bacc[k] = 0.0f;
+    bool ok = true;
+    // adds accumulator `grp` to the registers; uniform over the warp
+    auto flush = [&](int grp) {
+      const int b = grp & 1;
+      const bool waited = lane != 0 || mbar_wait(&tfull[b], (uint32_t)(grp >> 1) & 1, abort_flag, err, kWaitLimit);
+      if (!__all_sync(0xffffffffu, waited)) {
+        ok = false;
+        return;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx) {
+        float v[COUT];
+        tmem_ld<COUT>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 3 * kN + dx * kN + g * COUT), v);
+#pragma unroll
+        for (int c = 0; c < COUT; ++c) acc[dx][c] += v[c];
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[b]);
+    };
+    for (int i = 0; i < n + kWgLag && ok; ++i) {
+      if (i < n) {
+        const int s = i % kWgStages;
+        if (i >= kWgStages && lane == 0)
+          ok = mbar_wait(&empty[s], (uint32_t)(i / kWgStages - 1) & 1, abort_flag, err, kWaitLimit);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        // 32-bit divisions (the tiles fit, checked at launch); 64-bit ones took most of a tile's time
+        const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / (uint32_t)nseg;
+        const int x0 = (int)(t - by * (uint32_t)nseg) * kTileM, b = (int)(by / (uint32_t)npair);
+        const int y = 2 * (int)(by - (uint32_t)b * (uint32_t)npair);
+        const uint32_t st = smem0 + s * kWgStage;
+        // input rows y - 1 .. y + 2: pixels xp, xp + kXStep, ... of this thread's 8-channel group
+        const size_t img = (size_t)b * H;
+#pragma unroll
+        for (int row = 0; row < 4; ++row) {
+          const int yy = y + row - 1;
+          const bool iny = (unsigned)yy < (unsigned)H;
+          const uint16_t* src = X + ((img + (iny ? yy : 0)) * W + x0) * CIN + xc * 8;
+          const uint32_t dst = st + (row * XC + xc) * kWgPlane;
+#pragma unroll
+          for (int k = 0; k < kTileM / kXStep; ++k) {
+            const int px = xp + k * kXStep;  // halo pixel px is image column x0 + px - 1
+            const bool in = iny && (unsigned)(x0 + px - 1) < (unsigned)W;
+            cp_async16(dst + px * 16, in ? src + (px - 1) * CIN : X, in);
+          }
+        }
+        if (tid < 8 * XC) {  // the halo's last two pixels
+          const int row = tid / (2 * XC), px = kTileM + (tid / XC & 1), yy = y + row - 1;
+          const bool in = (unsigned)yy < (unsigned)H && x0 + px - 1 < W;
+          cp_async16(st + (row * XC + xc) * kWgPlane + px * 16,
+                     in ? X + ((img + yy) * W + (x0 + px - 1)) * CIN + xc * 8 : X, in);
+        }
+#pragma unroll
+        for (int row = 0; row < 2; ++row) {
+          const bool iny = y + row < H;
+          const uint16_t* src = Gr + ((img + (iny ? y + row : 0)) * W + x0) * COUT + gc * 8;
+          const uint32_t dst = st + (kWgXPlanes + row * GC + gc) * kWgPlane;
+#pragma unroll
+          for (int k = 0; k < kTileM / kGStep; ++k) {
+            const int px = gp + k * kGStep;
+            const bool in = iny && x0 + px < W;
+            cp_async16(dst + px * 16, in ? src + px * COUT : Gr, in);
+          }
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const int j = i - kWgLag;
+      if (j < 0) continue;
+      asm volatile("cp.async.wait_group %0;" ::"n"(kWgLag) : "memory");
+      const uint8_t* st = wg_smem + (j % kWgStages) * kWgStage;
+      // the gradient chunks this thread copied: always the same 8 channels
+#pragma unroll
+      for (int row = 0; row < 2; ++row)
+#pragma unroll
+        for (int k = 0; k < kTileM / kGStep; ++k) {
+          const uint4 w = *reinterpret_cast<const uint4*>(st + (kWgXPlanes + row * GC + gc) * kWgPlane +
+                                                          (gp + k * kGStep) * 16);
+          const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            bacc[2 * c] += bf_lo(u[c]);
+            bacc[2 * c + 1] += bf_hi(u[c]);
+          }
+        }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[j % kWgStages]);
+      if (j >= kWgGroup && j % kWgGroup == 1) flush(j / kWgGroup - 1);
+    }
+    // groups not flushed in the loop: the last one, and the one before it when the last holds a single tile
+    if (ok) {
+      const int last = (n - 1) / kWgGroup;
+      if (last >= 1 && (n - 1) % kWgGroup == 0) flush(last - 1);
+      if (ok) flush(last);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // nothing of this CTA is in flight when it leaves
+    if (ok && dy >= 0 && dy < 3) {
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+        for (int c = 0; c < COUT; ++c)
+          atomicAdd(dW + ((size_t)c * 9 + 3 * dy + dx) * CIN + ci, acc[dx][c]);
+    }
+    if (ok) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+#pragma unroll
+        for (int o = 16; o >= GC; o >>= 1) bacc[k] += __shfl_xor_sync(0xffffffffu, bacc[k], o);
+        if (lane < GC) atomicAdd(db + 8 * lane + k, bacc[k]);
+      }
+    }
+  } else if (lane == 0) {
+    // ---- MMA issuer -----------------------------------------------------------------------------
+    bool ok = true;
+    for (int j = 0; j < n && ok; ++j) {
+      const int s = j % kWgStages, grp = j / kWgGroup, b = grp & 1;
+      const bool first = j % kWgGroup == 0;
+      if (first && grp >= 2) ok = mbar_wait(&tempty[b], (uint32_t)((grp >> 1) - 1) & 1, abort_flag, err, kWaitLimit);
+      if (ok) ok = mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t xa = smem0 + s * kWgStage, ga = xa + kWgXPlanes * kWgPlane;
+      // MN-major, no swizzle: 128 bytes between groups of 8 pixels (K), one plane between 8-channel groups;
+      // an offset of 16 bytes is one unit of a descriptor's address
+      const uint64_t ad = desc_noswz(xa, 128, kWgPlane), bd = desc_noswz(ga, 128, kWgPlane);
+      const uint32_t acc = tmem + b * 3 * kN;
+#pragma unroll
+      for (int ks = 0; ks < kTileM / 16; ++ks)
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+          umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
+      umma_commit(&empty[s]);
+      if (j % kWgGroup == kWgGroup - 1 || j == n - 1) umma_commit(&tfull[b]);
+    }
+    // every tensor-core operation issued above completes before TMEM is freed
+    umma_commit(mdone);
+    mbar_drain(mdone, 0, err, kWaitLimit);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 8) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kWgTmemCols));
   }
 }
 
@@ -626,15 +813,15 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int COUT>
-int launch_wgrad(const uint16_t* X, const uint16_t* Gr, int B, int H, int W, float* dW, float* db, cudaStream_t s) {
-  const long long tiles = (long long)B * H * ((W + kTileM - 1) / kTileM);
-  const long long grid = std::min<long long>(tiles, 2LL * hr::sm_count());
+int launch_wgrad(const uint16_t* X, const uint16_t* Gr, int B, int H, int W, float* dW, float* db, int* err,
+                 cudaStream_t s) {
+  const long long tiles = (long long)B * ((H + 1) / 2) * ((W + kTileM - 1) / kTileM);
+  const long long grid = std::min<long long>(tiles, hr::sm_count());
   if (grid <= 0) return HR_OK;
-  const size_t smem = sizeof(float) * (3 * kHalo * CIN + kTileM * COUT);
-  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_kernel<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                   (int)cudaSharedmemCarveoutMaxShared));
-  wgrad_kernel<CIN, COUT><<<(unsigned)grid, (COUT / 4) * CIN, smem, s>>>(X, Gr, B, H, W, dW, db);
+  HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
+  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kWgSmem));
+  wgrad_tc_kernel<CIN, COUT><<<(unsigned)grid, kWgThreads, kWgSmem, s>>>(X, Gr, B, H, W, dW, db, err);
   HR_CUDA_TRY(cudaGetLastError());
   return HR_OK;
 }
@@ -836,11 +1023,11 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
     float* dW = n->d_g + n->woff[l];
     float* db = n->d_g + n->boff[l];
     if (ci == 16)
-      HR_TRY((launch_wgrad<16, 32>(n->d_act[l], g, B, H, W, dW, db, s)));
+      HR_TRY((launch_wgrad<16, 32>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
     else if (co == 16)
-      HR_TRY((launch_wgrad<32, 16>(n->d_act[l], g, B, H, W, dW, db, s)));
+      HR_TRY((launch_wgrad<32, 16>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
     else
-      HR_TRY((launch_wgrad<32, 32>(n->d_act[l], g, B, H, W, dW, db, s)));
+      HR_TRY((launch_wgrad<32, 32>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
     if (l == 0) break;
     ConvArgs b = base_args(n, B, H, W);
     b.in = g;

@@ -1,7 +1,7 @@
 """Learned artifact correction of half-view reconstructions (2.5D residual CNN).
 
 The network and its kernels live in libhelixrecon.so (hr_cnn_*): forward and
-backward-data convolutions on the tensor cores, weight gradients and Adam on
+backward convolutions and weight gradients on the tensor cores, Adam on
 the CUDA cores. This module holds the parameter initialisation, the training
 data the plain method produces from seeded phantoms, the training loop and
 the evaluation in HU.

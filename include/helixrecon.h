@@ -428,7 +428,7 @@ int hr_add_poisson_noise(float* d_proj, long long n, double I0, unsigned long lo
  * layers 3x3 (16->32, 6 x 32->32 with ReLU, 32->16 of which channel 0 is the
  * residual); output = centre slice + mu_w * residual. Forward and backward
  * data passes run on the tensor cores (BF16 operands, FP32 accumulation),
- * weight gradients on the CUDA cores; Adam on FP32 master parameters.
+ * and so do the weight gradients; Adam on FP32 master parameters.
  * Parameters: per layer W[co][tap][ci] (tap = 3*ky + kx) then b[co]. */
 typedef struct hr_cnn hr_cnn;
 size_t hr_cnn_param_count(void);

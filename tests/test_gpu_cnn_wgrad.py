@@ -1,0 +1,49 @@
+"""GPU tests of the tensor-core weight gradients at the edges of their tiling:
+two-row tiles (odd heights), 128-pixel strips (ragged widths), and enough tiles
+per CTA that both TMEM accumulators are flushed several times.
+
+Reference: the CPU oracle's backpropagation, which rounds to BF16 where the
+kernels store BF16, so what differs is the order of FP32 sums and the few
+activations whose rounding that order flips. A tile, tap or flush left out
+costs 10 % or more. Tolerance 3 %."""
+import numpy as np
+import pytest
+import torch
+
+from analyticalreconbigpatient_b200 import learned as L
+from analyticalreconbigpatient_b200.geometry import MU_WATER
+from conftest import rel_l2
+from oracle import cnn_oracle as C
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (1, 2, 129), (2, 7, 127), (1, 299, 513), (2, 310, 620)])
+def test_weight_gradients_vs_oracle(cuda, B, H, W):
+    rng = np.random.default_rng(H * 1000 + W)
+    params = L.init_params(3)
+    params[:] = params + 0.02 * rng.standard_normal(params.size).astype(np.float32)
+    g = torch.Generator(device=cuda).manual_seed(W)
+    u = torch.zeros((B, H, W, 16), device=cuda)
+    u[..., :5] = 0.3 * torch.randn((B, H, W, 5), device=cuda, generator=g)
+    ub = u.to(torch.bfloat16)
+    base = MU_WATER * (1 + 0.05 * torch.randn((B, H, W), device=cuda, generator=g))
+    target = base + 0.3 * MU_WATER * torch.randn((B, H, W), device=cuda, generator=g)
+    net = L.Corrector(params)
+    net.train_step(ub.view(torch.int16), base, target, lr=0.0)
+    got = net.grads()
+    net.check()
+    net.close()
+    _, ref = C.loss_and_grads(params, ub.float().cpu().numpy(), base.cpu().numpy(), target.cpu().numpy(), MU_WATER)
+    o = 0
+    for l, (ci, co) in enumerate(zip(L.CIN, L.COUT)):
+        n = 9 * ci * co
+        w, rw = got[o:o + n].reshape(co, 9, ci), ref[o:o + n].reshape(co, 9, ci)
+        b, rb = got[o + n:o + n + co], ref[o + n:o + n + co]
+        assert rel_l2(b, rb) < 3e-2, (l, "bias", rel_l2(b, rb))
+        for tap in range(9):
+            if np.linalg.norm(rw[:, tap]) > 0.05 * np.linalg.norm(rw):
+                assert rel_l2(w[:, tap], rw[:, tap]) < 3e-2, (l, tap, rel_l2(w[:, tap], rw[:, tap]))
+            else:  # taps that reach no pixel (a one-pixel image), or next to none
+                assert np.linalg.norm(w[:, tap] - rw[:, tap]) < 3e-2 * np.linalg.norm(rw)
+        o += n + co
