@@ -3,8 +3,10 @@
 // the stage on the current device's default stream, copies out and frees, as
 // the reference's thrust-based entries do -- but every CUDA call is checked.
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <memory>
+#include <thread>
 #include <vector>
 
 #include "hr_internal.h"
@@ -21,6 +23,42 @@ struct PlanGuard {
   ~PlanGuard() {
     if (p) Destroy(p);
   }
+};
+
+// Makes the pages of a caller's output buffer resident on helper threads while
+// the input is copied in and the kernels run. A result usually goes to memory
+// that was just allocated, and the copy out, one thread that stops at each
+// page's first fault, then takes twice its time (42 MB: about 10 ms instead of
+// 4). A page is touched by adding 0 to one of its bytes atomically, so the
+// contents stay as they are, also when the call fails. join() before anything
+// writes the buffer; without threads the copy out simply faults as before.
+class Prefault {
+ public:
+  Prefault(void* buf, size_t bytes) {
+    if (bytes < (size_t)4 << 20) return;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, buf) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
+      cudaGetLastError();  // not ordinary host memory: nothing to do
+      return;
+    }
+    const int n = 4;
+    auto* p = static_cast<unsigned char*>(buf);
+    try {
+      for (int i = 0; i < n; ++i)
+        t_.emplace_back([p, lo = bytes / n * i, hi = i + 1 < n ? bytes / n * (i + 1) : bytes] {
+          for (size_t o = lo; o < hi; o += 4096) __atomic_fetch_add(p + o, 0, __ATOMIC_RELAXED);
+        });
+    } catch (...) {
+    }
+  }
+  void join() {
+    for (std::thread& t : t_)
+      if (t.joinable()) t.join();
+  }
+  ~Prefault() { join(); }
+
+ private:
+  std::vector<std::thread> t_;
 };
 
 // View weight table of src/Parallel_FDK_Helical_3DWeighting.cpp:156-170, with
@@ -51,10 +89,12 @@ int bp_host(void* hvol, size_t vol_elem, const void* hfp, size_t fp_elem, const 
   const size_t nvol = (size_t)g.XN * g.YN * g.ZN;
   const size_t nfp = (size_t)g.YL * g.ZL * g.PN;
   hr::DeviceBuffer dvol, dfp;
+  Prefault pages(hvol, nvol * vol_elem);
   HR_TRY(dvol.alloc(nvol * vol_elem));
   HR_TRY(dfp.alloc(nfp * fp_elem));
   HR_CUDA_TRY(cudaMemcpy(dfp.ptr, hfp, nfp * fp_elem, cudaMemcpyHostToDevice));
   HR_TRY(hr_bp_execute(plan.p, dvol.ptr, dfp.ptr, nullptr));
+  pages.join();
   HR_CUDA_TRY(cudaMemcpy(hvol, dvol.ptr, nvol * vol_elem, cudaMemcpyDeviceToHost));
   return HR_OK;
 }
@@ -89,10 +129,12 @@ extern "C" int hr_rebin_host(float* out, const float* in, int YL, int ZL, int Vi
   HR_TRY(hr_rebin_plan_create(&plan.p, YL, ZL, ViewN, YLC, dYA, DeltaTheta, PLC, DeltaT, DeltaFai, SO));
   const size_t n = (size_t)YL * ZL * ViewN;
   hr::DeviceBuffer din, dout;
+  Prefault pages(out, n * sizeof(float));
   HR_TRY(din.alloc(n * sizeof(float)));
   HR_TRY(dout.alloc(n * sizeof(float)));
   HR_CUDA_TRY(cudaMemcpy(din.ptr, in, n * sizeof(float), cudaMemcpyHostToDevice));
   HR_TRY(hr_rebin_execute(plan.p, dout.as<float>(), din.as<float>(), nullptr));
+  pages.join();
   HR_CUDA_TRY(cudaMemcpy(out, dout.ptr, n * sizeof(float), cudaMemcpyDeviceToHost));
   return HR_OK;
 }
@@ -105,10 +147,12 @@ extern "C" int hr_filter_host(float* out, const float* in, int YL, int ZL, int V
   HR_TRY(hr_filter_plan_create(&plan.p, YL, ZL, ViewN, PLC, ZLC, dYL, dZL, SO));
   const size_t n = (size_t)YL * ZL * ViewN;
   hr::DeviceBuffer din, dout;
+  Prefault pages(out, n * sizeof(float));
   HR_TRY(din.alloc(n * sizeof(float)));
   HR_TRY(dout.alloc(n * sizeof(float)));
   HR_CUDA_TRY(cudaMemcpy(din.ptr, in, n * sizeof(float), cudaMemcpyHostToDevice));
   HR_TRY(hr_filter_execute(plan.p, dout.as<float>(), din.as<float>(), HR_LAYOUT_ROWS, 0, nullptr));
+  pages.join();
   HR_CUDA_TRY(cudaMemcpy(out, dout.ptr, n * sizeof(float), cudaMemcpyDeviceToHost));
   return HR_OK;
 }

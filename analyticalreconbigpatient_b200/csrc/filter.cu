@@ -34,6 +34,7 @@
 // straight to the output rows. Two shared-memory exchanges per pair of rows,
 // no block-wide barrier after set-up.
 #include <cmath>
+#include <complex>
 #include <cstdlib>
 #include <vector>
 
@@ -740,6 +741,33 @@ int launch2(const hr_filter_plan* p, float* out, const float* in, int view0, cud
 
 }  // namespace fft2k
 
+// Spectrum of a real, even, periodic sequence (N a power of two), divided by N:
+// a radix-2 transform in double. (Summing N cosines per frequency took 10.5 ms
+// of plan creation for N = 2048, which every host-pointer call pays.)
+std::vector<double> even_spectrum(const std::vector<double>& h) {
+  const size_t N = h.size();
+  std::vector<std::complex<double>> x(N), w(N / 2);
+  for (size_t t = 0; t < N / 2; ++t) w[t] = {std::cos(2.0 * M_PI * t / N), -std::sin(2.0 * M_PI * t / N)};
+  for (size_t i = 0, r = 0; i < N; ++i) {  // bit-reversed order
+    x[r] = h[i];
+    size_t bit = N >> 1;
+    for (; bit && (r & bit); bit >>= 1) r ^= bit;
+    r |= bit;
+  }
+  for (size_t len = 2; len <= N; len <<= 1)
+    for (size_t i = 0; i < N; i += len)
+      for (size_t k = 0; k < len / 2; ++k) {
+        const std::complex<double> u = x[i + k], v = x[i + k + len / 2], t = w[k * (N / len)];
+        const std::complex<double> vt(v.real() * t.real() - v.imag() * t.imag(),
+                                      v.real() * t.imag() + v.imag() * t.real());
+        x[i + k] = u + vt;
+        x[i + k + len / 2] = u - vt;
+      }
+  std::vector<double> s(N);
+  for (size_t k = 0; k < N; ++k) s[k] = x[k].real() / (double)N;
+  return s;
+}
+
 size_t smem_bytes(int log2N) {
   const size_t N = (size_t)1 << log2N;
   return 2 * kRowPairs * N * sizeof(float2) + N * sizeof(float2) + N * sizeof(float);
@@ -803,17 +831,9 @@ extern "C" int hr_filter_plan_create(hr_filter_plan** plan, int YL, int ZL, int 
     hs[n] = hn;
     if (n > 0) hs[N - n] = hn;
   }
-  std::vector<double> ct(N);
-  for (int t = 0; t < N; ++t) ct[t] = std::cos(2.0 * M_PI * t / N);
+  const std::vector<double> Hd = even_spectrum(hs);
   std::vector<float> H(N);
-  std::vector<double> Hd(N);
-  for (int k = 0; k < N; ++k) {
-    double acc = 0.0;
-    for (int n = 0; n < N; ++n)
-      if (hs[n] != 0.0) acc += hs[n] * ct[(size_t)k * n % N];
-    Hd[k] = acc / N;
-    H[k] = (float)Hd[k];
-  }
+  for (int k = 0; k < N; ++k) H[k] = (float)Hd[k];
   std::vector<float2> tw(N);
   for (int t = 0; t < N; ++t)
     tw[t] = make_float2((float)std::cos(2.0 * M_PI * t / N), (float)-std::sin(2.0 * M_PI * t / N));
