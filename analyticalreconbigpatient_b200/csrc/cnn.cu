@@ -7,26 +7,31 @@
 //   L1     : 16 -> 32, ReLU;   L2..L7: 32 -> 32, ReLU;   L8: 32 -> 16 (channel 0 used)
 //   output : centre slice (FP32, not rounded) + mu_w * L8 channel 0
 //
+// Inside the network activations and gradients are stored by planes: [B][H][C / 8][Wp][8]
+// BF16, a row of 16-byte pixel chunks per 8 channels with Wp = 128 ceil(W / 128) + 2 chunks,
+// one zero chunk before the image's first pixel and zeros after its last, so that a tile's
+// halo row is 130 contiguous chunks wherever it lies (rows above and below the image come
+// from a zero row). One untiled bulk copy brings such a row into shared memory, and an
+// epilogue's stores are contiguous over the warp. (With NHWC activations the same rows were
+// TMA boxes of 8 channels x 130 pixels, 16 bytes at a time, and bounded the kernels.) Every
+// epilogue writes its rows' zero chunks too, so nothing depends on what a buffer held.
+//
 // Convolutions run as implicit GEMMs on the 5th-generation tensor cores: one
 // tile is 128 output pixels of one image row (M = 128, TMEM lanes) by COUT
-// channels (N), K = 9 taps x CIN channels. A 3 x 130-pixel halo of the input
-// is staged in shared memory in the K-major no-swizzle layout (one plane of
-// 16-byte pixel chunks per 8-channel group; each plane is one TMA box of 8
-// channels x 130 pixels, zero-filled outside the image), so the A operand of
-// tap (dy, dx) is the same buffer seen from another 16-byte-aligned start
-// address: every input pixel is loaded once per tile and nine descriptor
-// offsets replace an im2col copy. The weights (B operand) stay in shared
-// memory for the CTA's life. Persistent, warp-specialised CTAs: warp 0 issues
-// the TMA loads into a 3-stage halo ring, warp 1 issues the 9*CIN/16
-// tcgen05.mma of a tile into one of two TMEM accumulators, warps 2-5 read the
-// other accumulator and run the epilogue (bias + ReLU + BF16 store; gradient
-// masking by the forward activation; fused residual + loss + output
-// gradient), so loads, MMAs and stores of consecutive tiles overlap. Every
-// mbarrier wait is bounded and sets an error flag when it gives up. The
-// backward data pass is the same kernel with the weights transposed and
-// flipped. Weight gradients are a second tensor-core kernel that contracts over
-// the pixels (wgrad_tc_kernel).
-#include <cuda.h>
+// channels (N), K = 9 taps x CIN channels. The input rows lie in shared memory
+// in the K-major no-swizzle layout (one plane of 16-byte pixel chunks per
+// 8-channel group), so the A operand of tap (dy, dx) is the same buffer seen
+// from another 16-byte-aligned start address: nine descriptor offsets replace
+// an im2col copy. The weights (B operand) stay in shared memory for the CTA's
+// life. Persistent, warp-specialised CTAs: warp 0 issues the copies into a
+// ring of input rows, warp 1 issues the 9*CIN/16 tcgen05.mma of a tile into
+// one of two TMEM accumulators, warps 2-5 read the other accumulator and run
+// the epilogue (bias + ReLU + BF16 store; gradient masking by the forward
+// activation; fused residual + loss + output gradient), so loads, MMAs and
+// stores of consecutive tiles overlap. Every mbarrier wait is bounded and sets
+// an error flag when it gives up. The backward data pass is the same kernel
+// with the weights transposed and flipped. Weight gradients are a second
+// tensor-core kernel that contracts over the pixels (wgrad_tc_kernel).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -40,8 +45,8 @@ namespace {
 
 constexpr int kTileM = 128;                  // output pixels per tile (one row segment)
 constexpr int kHalo = kTileM + 2;            // halo pixels per row
-constexpr int kBox = kHalo * 16;             // bytes of one TMA box: 8 channels x 130 pixels
-constexpr int kPlane = 17 * 128;             // plane stride: one box, 128-byte aligned
+constexpr int kBox = kHalo * 16;             // bytes of one halo row: 130 pixel chunks of 8 channels
+constexpr int kPlane = 17 * 128;             // plane stride: one halo row, 128-byte aligned
 constexpr int kRing = 6;                     // halo ring: input rows in flight
 constexpr int kThreads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 constexpr int kTmemCols = 64;                // two 32-column accumulators
@@ -138,14 +143,17 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// 4D tiled TMA load (no multicast): box {8 channels, 130 pixels, 1 row, 1 image}.
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c, int x, int y,
-                                            int b) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
-      "[%2];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c), "r"(x), "r"(y), "r"(b)
-      : "memory");
+// Untiled bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned), reported to `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// Chunks of a padded row, and the chunk offset of channel group c of image row (b, y) (G groups).
+__host__ __device__ constexpr int padded_width(int W) { return (W + kTileM - 1) / kTileM * kTileM + 2; }
+__device__ __forceinline__ size_t plane_row(int b, int H, int y, int G, int c, int Wp) {
+  return (((size_t)b * H + y) * G + c) * Wp;
 }
 
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -185,12 +193,12 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float (&v)[32]) {
 }
 
 struct ConvArgs {
-  CUtensorMap in_map;    // the input as a 4D tensor {CIN, W, H, B} of BF16, box {8, 130, 1, 1}
-  const uint16_t* in;    // NHWC BF16 [B][H][W][CIN]
+  const uint4* in;       // input planes, CIN / 8 groups
+  const uint4* zero;     // kHalo zero chunks
   const uint16_t* wimg;  // B operand image [9*CIN/8][COUT][8] BF16
   const float* bias;     // [COUT] (EPI_RELU, EPI_LOSS, EPI_RESID)
-  uint16_t* out;         // NHWC BF16 [B][H][W][COUT] (EPI_RELU, EPI_MASK); output gradient (EPI_LOSS)
-  const uint16_t* mask;  // NHWC BF16 [B][H][W][COUT]: forward activation whose > 0 passes the gradient (EPI_MASK)
+  uint4* out;            // output planes, COUT / 8 groups (EPI_RELU, EPI_MASK); output gradient (EPI_LOSS)
+  const uint4* mask;     // planes of the forward activation whose > 0 passes the gradient (EPI_MASK)
   // residual epilogues: element (b, y, x) of base/target/pred at b*sb + (y*W + x)*sp
   const float* base;
   const float* target;   // EPI_LOSS
@@ -199,7 +207,7 @@ struct ConvArgs {
   float scale;           // mu_w: pred = base + scale * r
   float grad_scale;      // EPI_LOSS: d loss / d r = grad_scale * (pred - target) / scale
   float* loss;           // EPI_LOSS: accumulates sum ((pred - target) / scale)^2
-  int B, H, W;
+  int B, H, W, Wp;
   int rows_per_unit;     // output rows a CTA computes down one 128-pixel column strip
   int* err;
   int stall_row;         // test hook: the CTA's input row of this index is never loaded (-1: none)
@@ -210,39 +218,45 @@ struct ConvArgs {
 template <int COUT, int EPI>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v)[COUT], const float* bias_s, int b,
                                               int y, int x, int lane) {
-  const bool valid = x < a.W;
-  const size_t pix = ((size_t)b * a.H + y) * a.W + x;
+  const bool valid = x < a.W;  // pixels beyond the image are stored as zeros
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const size_t row = plane_row(b, a.H, y, COUT / 8, 0, a.Wp);
+  if constexpr (EPI != EPI_RESID) {  // the zero chunks before the first and after the last tile pixel
+    if (x == 0 || x == a.Wp - 3) {
+#pragma unroll
+      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + (x == 0 ? 0 : a.Wp - 1)] = zero;
+    }
+  }
   if constexpr (EPI == EPI_RELU) {
-    if (valid) {
-      uint4* o = reinterpret_cast<uint4*>(a.out + pix * COUT);
+    uint4* o = a.out + row + x + 1;
 #pragma unroll
-      for (int c = 0; c < COUT / 8; ++c) {
-        float u[8];
+    for (int c = 0; c < COUT / 8; ++c) {
+      float u[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) u[j] = fmaxf(v[8 * c + j] + bias_s[8 * c + j], 0.0f);
-        o[c] = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]), pack2(u[6], u[7]));
-      }
+      for (int j = 0; j < 8; ++j) u[j] = fmaxf(v[8 * c + j] + bias_s[8 * c + j], 0.0f);
+      o[(size_t)c * a.Wp] = valid ? make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]),
+                                               pack2(u[6], u[7]))
+                                  : zero;
     }
   } else if constexpr (EPI == EPI_MASK) {
-    if (valid) {
-      const uint4* m = reinterpret_cast<const uint4*>(a.mask + pix * COUT);
-      uint4* o = reinterpret_cast<uint4*>(a.out + pix * COUT);
+    const uint4* m = a.mask + row + x + 1;
+    uint4* o = a.out + row + x + 1;
 #pragma unroll
-      for (int c = 0; c < COUT / 8; ++c) {
-        const uint4 mv = __ldg(m + c);
-        const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
-        float u[8];
+    for (int c = 0; c < COUT / 8; ++c) {
+      const uint4 mv = __ldg(m + (size_t)c * a.Wp);  // zero beyond the image: masks those pixels too
+      const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
+      float u[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          u[2 * j] = bf_lo(mw[j]) > 0.0f ? v[8 * c + 2 * j] : 0.0f;
-          u[2 * j + 1] = bf_hi(mw[j]) > 0.0f ? v[8 * c + 2 * j + 1] : 0.0f;
-        }
-        o[c] = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]), pack2(u[6], u[7]));
+      for (int j = 0; j < 4; ++j) {
+        u[2 * j] = bf_lo(mw[j]) > 0.0f ? v[8 * c + 2 * j] : 0.0f;
+        u[2 * j + 1] = bf_hi(mw[j]) > 0.0f ? v[8 * c + 2 * j + 1] : 0.0f;
       }
+      o[(size_t)c * a.Wp] = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]), pack2(u[6], u[7]));
     }
   } else {
     const float r = v[0] + bias_s[0];
     float e2 = 0.0f;
+    [[maybe_unused]] uint4 g0 = zero;
     if (valid) {
       const size_t off = (size_t)b * a.sb + ((size_t)y * a.W + x) * a.sp;
       const float pr = a.base[off] + a.scale * r;
@@ -252,13 +266,12 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
         if (a.pred) a.pred[off] = pr;
         const float e = (pr - a.target[off]) / a.scale;
         e2 = e * e;
-        uint4* o = reinterpret_cast<uint4*>(a.out + pix * COUT);
-        o[0] = make_uint4(pack2(a.grad_scale * e, 0.0f), 0u, 0u, 0u);
-#pragma unroll
-        for (int c = 1; c < COUT / 8; ++c) o[c] = make_uint4(0u, 0u, 0u, 0u);
+        g0 = make_uint4(pack2(a.grad_scale * e, 0.0f), 0u, 0u, 0u);
       }
     }
     if constexpr (EPI == EPI_LOSS) {
+#pragma unroll
+      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + x + 1] = c == 0 ? g0 : zero;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
       if (lane == 0 && e2 != 0.0f) atomicAdd(a.loss, e2);
@@ -267,8 +280,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 }
 
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant__ ConvArgs a) {
-  constexpr int G = CIN / 8;                 // 8-channel groups (TMA boxes per input row)
+__global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_constant__ ConvArgs a) {
+  constexpr int G = CIN / 8;                 // 8-channel groups (copies per input row)
   constexpr int kRow = G * kPlane;           // bytes of one input row (130 pixels)
   constexpr int kWBytes = 9 * CIN * COUT * 2;
   constexpr int kKSteps = 9 * CIN / 16;
@@ -323,7 +336,7 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
   const int nchunk = (a.H + rpu - 1) / rpu;
   const long long units = (long long)a.B * nseg * nchunk;
   if (warp == 0) {
-    // ---- producer: input rows of each unit into the ring, G boxes per row --------------------
+    // ---- producer: input rows of each unit into the ring, G halo rows each -------------------
     if (lane == 0) {
       int h = 0;  // input rows loaded by this CTA
       int last_h[kRing];
@@ -342,8 +355,11 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
           if (h == a.stall_row) continue;  // test hook: this row's slot is never filled
           last_h[s] = h;
           mbar_expect_tx(&full[s], kTxBytes);
+          const int y = y0 - 1 + j;
+          const bool in = y >= 0 && y < a.H;
+          const uint4* src = in ? a.in + plane_row(b, a.H, y, G, 0, a.Wp) + seg * kTileM : a.zero;
           for (int g = 0; g < G; ++g)
-            tma_load_4d(smem_a + s * kRow + g * kPlane, &a.in_map, &full[s], g * 8, seg * kTileM - 1, y0 - 1 + j, b);
+            bulk_load(smem_a + s * kRow + g * kPlane, src + (in ? (size_t)g * a.Wp : 0), kBox, &full[s]);
         }
       }
       // every issued copy lands before the CTA exits (after an abort nobody consumes them)
@@ -430,16 +446,14 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
 // (K = 16 pixels) give every D_dx[(r, ci)][(g, co)]; the combinations with 0 <= r - g <= 2
 // are dW at dy = r - g, six of eight. Shared memory holds one plane of 16-byte pixel chunks
 // per 8 channels (the no-swizzle layout: planes along M / N, groups of 8 pixels along K),
-// filled by 16-byte asynchronous copies with zeros outside the image; planes are 2080 bytes
-// apart, so the four lanes that copy one pixel write different banks.
+// filled by one bulk copy per row and group.
 //
-// Warps 0-7 copy the tiles through a four-stage ring, add up their own gradient chunks for
-// db, and every kWgGroup tiles add the finished accumulator (one of two in TMEM) to FP32
-// registers with rounding to nearest, so that the tensor core's own accumulation, which
-// truncates, runs over 32 steps at most (left to run over a CTA's whole share it shrinks the
-// gradients by 1.1e-5; over four tiles by 4e-7); warp 8 issues the MMAs. A warp reads its
-// TMEM lane quarter (row r for 32 input channels) for one gradient row. Barriers are waited
-// on and arrived at by one lane per warp. Every wait is bounded.
+// Warp 9 issues the copies into a four-stage ring, warp 8 the MMAs; warps 0-7 sum each
+// stage's gradient chunks for db, and every kWgGroup tiles add the finished accumulator (one
+// of two in TMEM) to FP32 registers with rounding to nearest, so that the tensor core's own
+// accumulation, which truncates, runs over 32 steps at most (left to run over a CTA's whole
+// share it shrinks the gradients by 1.1e-5; over four tiles by 4e-7). A warp reads its TMEM
+// lane quarter (row r for 32 input channels) for one gradient row. Every wait is bounded.
 //
 // The CUDA-core kernel this replaced (36 FP32 accumulators per thread, 13 shared-memory
 // reads per 36 FMAs) took 1.40 ms per 32 -> 32 layer of 8 x 512 x 512, 11.0 of the 12.6 ms
@@ -449,23 +463,18 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
 // fewer MMAs, flushes or bias sums change nothing).
 constexpr int kWgStages = 4;
 constexpr int kWgGroup = 4;                          // tiles accumulated in TMEM before a flush
-constexpr int kWgPlane = kHalo * 16;                 // bytes between planes (2080: 32 mod 128)
+constexpr int kWgPlane = kHalo * 16;                 // bytes between planes
 constexpr int kWgXPlanes = 16, kWgGPlanes = 8;       // M = 128, N <= 64
 constexpr int kWgStage = (kWgXPlanes + kWgGPlanes) * kWgPlane;
-constexpr int kWgProducers = 256;                    // warps 0-7
-constexpr int kWgThreads = kWgProducers + 32;
-constexpr int kWgLag = 2;                            // tiles a copy is given to land
+constexpr int kWgWorkers = 8;                        // warps 0-7: bias sums and flushes
+constexpr int kWgThreads = 32 * (kWgWorkers + 2);
 constexpr int kWgTmemCols = 512;
 constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256;
 
-// 16-byte asynchronous copy to shared memory; zeros if !valid (src is not read then).
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t* __restrict__ X,
-                                                                 const uint16_t* __restrict__ Gr, int B, int H, int W,
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __restrict__ X,
+                                                                 const uint4* __restrict__ Gr,
+                                                                 const uint4* __restrict__ zero, int B, int H, int W,
                                                                  float* __restrict__ dW, float* __restrict__ db,
                                                                  int* __restrict__ err) {
   constexpr int XC = CIN / 8, GC = COUT / 8;        // 16-byte chunks per pixel
@@ -474,31 +483,32 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
   constexpr uint32_t kIdesc = idesc_bf16(kN) | (1u << 15) | (1u << 16);
   extern __shared__ __align__(128) uint8_t wg_smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(wg_smem + kWgStages * kWgStage);
-  uint64_t* empty = full + kWgStages;
+  uint64_t* empty = full + kWgStages;    // the MMAs have read the stage and the workers summed it
   uint64_t* tfull = empty + kWgStages;   // [2] accumulator complete
   uint64_t* tempty = tfull + 2;          // [2] accumulator read out
   uint64_t* mdone = tempty + 2;          // the MMA issuer's last commit
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // planes no copy fills (16 input channels) are read as rows of D that nobody uses
-  for (int i = tid; i < kWgStages * kWgStage / 16; i += kWgThreads)
-    reinterpret_cast<uint4*>(wg_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if constexpr (XC * 4 < kWgXPlanes) {  // planes no copy fills are read as rows of D that nobody uses
+    for (int i = tid; i < kWgStages * kWgStage / 16; i += kWgThreads)
+      reinterpret_cast<uint4*>(wg_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
   if (tid == 0) {
     for (int s = 0; s < kWgStages; ++s) {
-      mbar_init(&full[s], kWgProducers / 32);
-      mbar_init(&empty[s], 1);
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1 + kWgWorkers);
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&tfull[s], 1);
-      mbar_init(&tempty[s], kWgProducers / 32);
+      mbar_init(&tempty[s], kWgWorkers);
     }
     mbar_init(mdone, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 8) {
+  if (warp == kWgWorkers) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(kWgTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -509,19 +519,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
   const uint32_t tmem = *tmem_slot;
   const uint32_t smem0 = smem_u32(wg_smem);
 
-  const int nseg = (W + kTileM - 1) / kTileM, npair = (H + 1) / 2;
-  const long long tiles = (long long)B * npair * nseg;
-  const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // this CTA's tiles (grid <= tiles)
+  const int Wp = padded_width(W);
+  const uint32_t nseg = (uint32_t)(Wp - 2) / kTileM, npair = (uint32_t)(H + 1) / 2;
+  const uint32_t tiles = (uint32_t)B * npair * nseg;                                 // < 2^31, checked at launch
+  const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);             // this CTA's (grid <= tiles)
 
-  if (warp < 8) {
-    // ---- copies, bias sums and flushes ---------------------------------------------------------
+  if (warp < kWgWorkers) {
+    // ---- bias sums and flushes -------------------------------------------------------------------
     const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter and gradient row this warp flushes
     const int m = q * 32 + lane;            // row of D
     const int r = m / CIN, ci = m - r * CIN, dy = r - g;
-    // copies: this thread's 8-channel group and first pixel of the input and the gradient rows
-    constexpr int kXStep = kWgProducers / XC, kGStep = kWgProducers / GC;
-    static_assert(kTileM % kXStep == 0 && kTileM % kGStep == 0, "whole passes over a row");
-    const int xc = tid % XC, xp = tid / XC, gc = tid % GC, gp = tid / GC;
     float acc[3][COUT];
 #pragma unroll
     for (int dx = 0; dx < 3; ++dx)
@@ -551,66 +558,22 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[b]);
     };
-    for (int i = 0; i < n + kWgLag && ok; ++i) {
-      if (i < n) {
-        const int s = i % kWgStages;
-        if (i >= kWgStages && lane == 0)
-          ok = mbar_wait(&empty[s], (uint32_t)(i / kWgStages - 1) & 1, abort_flag, err, kWaitLimit);
-        if (!__all_sync(0xffffffffu, ok)) {
-          ok = false;
-          break;
-        }
-        // 32-bit divisions (the tiles fit, checked at launch); 64-bit ones took most of a tile's time
-        const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / (uint32_t)nseg;
-        const int x0 = (int)(t - by * (uint32_t)nseg) * kTileM, b = (int)(by / (uint32_t)npair);
-        const int y = 2 * (int)(by - (uint32_t)b * (uint32_t)npair);
-        const uint32_t st = smem0 + s * kWgStage;
-        // input rows y - 1 .. y + 2: pixels xp, xp + kXStep, ... of this thread's 8-channel group
-        const size_t img = (size_t)b * H;
-#pragma unroll
-        for (int row = 0; row < 4; ++row) {
-          const int yy = y + row - 1;
-          const bool iny = (unsigned)yy < (unsigned)H;
-          const uint16_t* src = X + ((img + (iny ? yy : 0)) * W + x0) * CIN + xc * 8;
-          const uint32_t dst = st + (row * XC + xc) * kWgPlane;
-#pragma unroll
-          for (int k = 0; k < kTileM / kXStep; ++k) {
-            const int px = xp + k * kXStep;  // halo pixel px is image column x0 + px - 1
-            const bool in = iny && (unsigned)(x0 + px - 1) < (unsigned)W;
-            cp_async16(dst + px * 16, in ? src + (px - 1) * CIN : X, in);
-          }
-        }
-        if (tid < 8 * XC) {  // the halo's last two pixels
-          const int row = tid / (2 * XC), px = kTileM + (tid / XC & 1), yy = y + row - 1;
-          const bool in = (unsigned)yy < (unsigned)H && x0 + px - 1 < W;
-          cp_async16(st + (row * XC + xc) * kWgPlane + px * 16,
-                     in ? X + ((img + yy) * W + (x0 + px - 1)) * CIN + xc * 8 : X, in);
-        }
-#pragma unroll
-        for (int row = 0; row < 2; ++row) {
-          const bool iny = y + row < H;
-          const uint16_t* src = Gr + ((img + (iny ? y + row : 0)) * W + x0) * COUT + gc * 8;
-          const uint32_t dst = st + (kWgXPlanes + row * GC + gc) * kWgPlane;
-#pragma unroll
-          for (int k = 0; k < kTileM / kGStep; ++k) {
-            const int px = gp + k * kGStep;
-            const bool in = iny && x0 + px < W;
-            cp_async16(dst + px * 16, in ? src + px * COUT : Gr, in);
-          }
-        }
+    // a worker sums one channel group: group tid % GC, pixels tid / GC, + 256 / GC, ... of both gradient rows
+    const int gc = tid % GC, gp = tid / GC;
+    for (int j = 0; j < n && ok; ++j) {
+      const int s = j % kWgStages;
+      const bool waited =
+          lane != 0 || mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
+      if (!__all_sync(0xffffffffu, waited)) {
+        ok = false;
+        break;
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      const int j = i - kWgLag;
-      if (j < 0) continue;
-      asm volatile("cp.async.wait_group %0;" ::"n"(kWgLag) : "memory");
-      const uint8_t* st = wg_smem + (j % kWgStages) * kWgStage;
-      // the gradient chunks this thread copied: always the same 8 channels
+      const uint8_t* st = wg_smem + s * kWgStage + kWgXPlanes * kWgPlane;
 #pragma unroll
       for (int row = 0; row < 2; ++row)
 #pragma unroll
-        for (int k = 0; k < kTileM / kGStep; ++k) {
-          const uint4 w = *reinterpret_cast<const uint4*>(st + (kWgXPlanes + row * GC + gc) * kWgPlane +
-                                                          (gp + k * kGStep) * 16);
+        for (int px = 0; px < kTileM; px += 32 * kWgWorkers / GC) {
+          const uint4 w = *reinterpret_cast<const uint4*>(st + (row * GC + gc) * kWgPlane + (gp + px) * 16);
           const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -618,9 +581,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
             bacc[2 * c + 1] += bf_hi(u[c]);
           }
         }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&full[j % kWgStages]);
+      if (lane == 0) mbar_arrive(&empty[s]);
       if (j >= kWgGroup && j % kWgGroup == 1) flush(j / kWgGroup - 1);
     }
     // groups not flushed in the loop: the last one, and the one before it when the last holds a single tile
@@ -629,7 +591,6 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
       if (last >= 1 && (n - 1) % kWgGroup == 0) flush(last - 1);
       if (ok) flush(last);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");  // nothing of this CTA is in flight when it leaves
     if (ok && dy >= 0 && dy < 3) {
 #pragma unroll
       for (int dx = 0; dx < 3; ++dx)
@@ -645,36 +606,68 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint16_t*
         if (lane < GC) atomicAdd(db + 8 * lane + k, bacc[k]);
       }
     }
-  } else if (lane == 0) {
+  } else if (warp == kWgWorkers) {
     // ---- MMA issuer -----------------------------------------------------------------------------
-    bool ok = true;
-    for (int j = 0; j < n && ok; ++j) {
-      const int s = j % kWgStages, grp = j / kWgGroup, b = grp & 1;
-      const bool first = j % kWgGroup == 0;
-      if (first && grp >= 2) ok = mbar_wait(&tempty[b], (uint32_t)((grp >> 1) - 1) & 1, abort_flag, err, kWaitLimit);
-      if (ok) ok = mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t xa = smem0 + s * kWgStage, ga = xa + kWgXPlanes * kWgPlane;
-      // MN-major, no swizzle: 128 bytes between groups of 8 pixels (K), one plane between 8-channel groups;
-      // an offset of 16 bytes is one unit of a descriptor's address
-      const uint64_t ad = desc_noswz(xa, 128, kWgPlane), bd = desc_noswz(ga, 128, kWgPlane);
-      const uint32_t acc = tmem + b * 3 * kN;
+    if (lane == 0) {
+      bool ok = true;
+      for (int j = 0; j < n && ok; ++j) {
+        const int s = j % kWgStages, grp = j / kWgGroup, b = grp & 1;
+        const bool first = j % kWgGroup == 0;
+        if (first && grp >= 2)
+          ok = mbar_wait(&tempty[b], (uint32_t)((grp >> 1) - 1) & 1, abort_flag, err, kWaitLimit);
+        if (ok) ok = mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t xa = smem0 + s * kWgStage, ga = xa + kWgXPlanes * kWgPlane;
+        // MN-major, no swizzle: 128 bytes between groups of 8 pixels (K), one plane between 8-channel groups;
+        // an offset of 16 bytes is one unit of a descriptor's address
+        const uint64_t ad = desc_noswz(xa, 128, kWgPlane), bd = desc_noswz(ga, 128, kWgPlane);
+        const uint32_t acc = tmem + b * 3 * kN;
 #pragma unroll
-      for (int ks = 0; ks < kTileM / 16; ++ks)
+        for (int ks = 0; ks < kTileM / 16; ++ks)
 #pragma unroll
-        for (int dx = 0; dx < 3; ++dx)
-          umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
-      umma_commit(&empty[s]);
-      if (j % kWgGroup == kWgGroup - 1 || j == n - 1) umma_commit(&tfull[b]);
+          for (int dx = 0; dx < 3; ++dx)
+            umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
+        umma_commit(&empty[s]);
+        if (j % kWgGroup == kWgGroup - 1 || j == n - 1) umma_commit(&tfull[b]);
+      }
+      // every tensor-core operation issued above completes before TMEM is freed
+      umma_commit(mdone);
+      mbar_drain(mdone, 0, err, kWaitLimit);
     }
-    // every tensor-core operation issued above completes before TMEM is freed
-    umma_commit(mdone);
-    mbar_drain(mdone, 0, err, kWaitLimit);
+  } else if (lane == 0) {
+    // ---- copies: halo rows of input rows y - 1 .. y + 2, tile rows of gradient rows y, y + 1 --------
+    int issued = 0;
+    for (int i = 0; i < n; ++i) {
+      const int s = i % kWgStages;
+      if (i >= kWgStages && !mbar_wait(&empty[s], (uint32_t)(i / kWgStages - 1) & 1, abort_flag, err, kWaitLimit))
+        break;
+      const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / nseg;
+      const int x0 = (int)(t - by * nseg) * kTileM, b = (int)(by / npair), y = 2 * (int)(by - (uint32_t)b * npair);
+      const uint32_t st = smem0 + s * kWgStage;
+      mbar_expect_tx(&full[s], 4 * XC * kBox + 2 * GC * kTileM * 16);
+      for (int row = 0; row < 4; ++row) {
+        const int yy = y + row - 1;
+        const bool in = yy >= 0 && yy < H;
+        const uint4* src = in ? X + plane_row(b, H, yy, XC, 0, Wp) + x0 : zero;
+        for (int c = 0; c < XC; ++c)
+          bulk_load(st + (row * XC + c) * kWgPlane, src + (in ? (size_t)c * Wp : 0), kBox, &full[s]);
+      }
+      for (int row = 0; row < 2; ++row) {
+        const bool in = y + row < H;
+        const uint4* src = in ? Gr + plane_row(b, H, y + row, GC, 0, Wp) + x0 + 1 : zero;
+        for (int c = 0; c < GC; ++c)
+          bulk_load(st + (kWgXPlanes + row * GC + c) * kWgPlane, src + (in ? (size_t)c * Wp : 0), kTileM * 16, &full[s]);
+      }
+      issued = i + 1;
+    }
+    // every issued copy lands before the CTA exits (after an abort nobody consumes them)
+    for (int i = issued > kWgStages ? issued - kWgStages : 0; i < issued; ++i)
+      mbar_drain(&full[i % kWgStages], (uint32_t)(i / kWgStages) & 1, err, kWaitLimit);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 8) {
+  if (warp == kWgWorkers) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kWgTmemCols));
   }
@@ -738,39 +731,59 @@ __global__ void pack_input_kernel(uint16_t* __restrict__ out, const float* __res
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-int get_encoder(EncodeTiledFn* fn) {
-  static EncodeTiledFn cached = nullptr;
-  if (!cached) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    HR_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
-    if (q != cudaDriverEntryPointSuccess || p == nullptr)
-      return hr::fail(HR_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
-    cached = reinterpret_cast<EncodeTiledFn>(p);
+// The same input as planes (two groups: 8 channels of which 5 are used, 8 of zeros) for the
+// network itself. A CTA takes 32 padded pixels of one image row and 32 slices: it reads each
+// pixel's 36 consecutive slices together (the volume's fastest axis) and writes rows of pixels.
+constexpr int kPackPx = 32, kPackZ = 32;
+__global__ void __launch_bounds__(256) pack_planes_kernel(uint4* __restrict__ out, const float* __restrict__ vol, int XN,
+                                                          int YN, int ZN, int z0, int nz, float inv_mu, int Wp) {
+  __shared__ float t[kPackPx][kPackZ + 5];
+  const int px0 = blockIdx.x * kPackPx, y = blockIdx.y, s0 = blockIdx.z * kPackZ;
+  for (int i = threadIdx.x; i < kPackPx * (kPackZ + 4); i += 256) {
+    const int p = i / (kPackZ + 4), k = i - p * (kPackZ + 4);
+    const int x = px0 + p - 1, z = min(max(z0 + s0 + k - 2, 0), ZN - 1);
+    if (x >= 0 && x < XN && s0 + k < nz + 4) t[p][k] = vol[((size_t)y * XN + x) * ZN + z];
   }
-  *fn = cached;
-  return HR_OK;
+  __syncthreads();
+  const int p = threadIdx.x & (kPackPx - 1), px = px0 + p, x = px - 1;
+  if (px >= Wp) return;
+  for (int k = threadIdx.x / kPackPx; k < kPackZ && s0 + k < nz; k += 256 / kPackPx) {
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    if (x >= 0 && x < XN) {
+      float u[5];
+#pragma unroll
+      for (int c = 0; c < 5; ++c) u[c] = t[p][k + c] * inv_mu - 1.0f;
+      w = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], 0.0f), 0u);
+    }
+    const size_t o = plane_row(s0 + k, YN, y, 2, 0, Wp) + px;
+    out[o] = w;
+    out[o + Wp] = make_uint4(0u, 0u, 0u, 0u);
+  }
 }
 
-// The NHWC BF16 activation [B][H][W][C] as a 4D TMA tensor {C, W, H, B}; box
-// {8, 130, 1, 1}; out-of-range elements read as zero (the conv padding).
-int make_act_map(CUtensorMap* map, const void* base, int C, int B, int H, int W) {
-  EncodeTiledFn enc;
-  HR_TRY(get_encoder(&enc));
-  HR_REQUIRE(((uintptr_t)base & 15) == 0, "conv: activation must be 16-byte aligned");
-  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-  const cuuint32_t box[4] = {8, (cuuint32_t)kHalo, 1, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return hr::fail(HR_ERR_CUDA, "cuTensorMapEncodeTiled (activation) failed (%d)", (int)r);
-  return HR_OK;
+// A caller's NHWC input [rows][W][16] as planes (ALIGNED: it starts on a 16-byte boundary).
+template <bool ALIGNED>
+__global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* __restrict__ in, long long rows, int W,
+                                      int Wp) {
+  const long long total = rows * Wp;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / Wp;
+    const int px = (int)(i - r * Wp), x = px - 1;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (x >= 0 && x < W) {
+        const uint16_t* src = in + (r * W + x) * 16 + c * 8;
+        if constexpr (ALIGNED)
+          w = __ldg(reinterpret_cast<const uint4*>(src));
+        else
+          w = make_uint4(src[0] | (uint32_t)src[1] << 16, src[2] | (uint32_t)src[3] << 16,
+                         src[4] | (uint32_t)src[5] << 16, src[6] | (uint32_t)src[7] << 16);
+      }
+      out[(r * 2 + c) * Wp + px] = w;
+    }
+  }
 }
 
 // Dynamic shared memory of a conv CTA: input-row ring + weights + barriers + alignment slack.
@@ -782,7 +795,6 @@ constexpr size_t conv_smem() {
 template <int CIN, int COUT, int EPI>
 int launch_conv(ConvArgs& a, cudaStream_t s) {
   const size_t smem = conv_smem<CIN, COUT>();
-  HR_TRY(make_act_map(&a.in_map, a.in, CIN, a.B, a.H, a.W));
   HR_CUDA_TRY(cudaFuncSetAttribute(conv_tc_kernel<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
   // the largest shared-memory carveout, so that several CTAs (input-row rings) fit on an SM
@@ -813,15 +825,15 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
 }
 
 template <int CIN, int COUT>
-int launch_wgrad(const uint16_t* X, const uint16_t* Gr, int B, int H, int W, float* dW, float* db, int* err,
-                 cudaStream_t s) {
+int launch_wgrad(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
+                 int* err, cudaStream_t s) {
   const long long tiles = (long long)B * ((H + 1) / 2) * ((W + kTileM - 1) / kTileM);
   const long long grid = std::min<long long>(tiles, hr::sm_count());
   if (grid <= 0) return HR_OK;
   HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
   HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kWgSmem));
-  wgrad_tc_kernel<CIN, COUT><<<(unsigned)grid, kWgThreads, kWgSmem, s>>>(X, Gr, B, H, W, dW, db, err);
+  wgrad_tc_kernel<CIN, COUT><<<(unsigned)grid, kWgThreads, kWgSmem, s>>>(X, Gr, zero, B, H, W, dW, db, err);
   HR_CUDA_TRY(cudaGetLastError());
   return HR_OK;
 }
@@ -833,10 +845,11 @@ struct hr_cnn {
   size_t woff[kLayers], boff[kLayers], nparam = 0;
   float *d_p = nullptr, *d_g = nullptr, *d_m = nullptr, *d_v = nullptr;
   uint16_t *d_wf[kLayers] = {}, *d_wb[kLayers] = {};  // BF16 operand images (forward, backward)
-  // activations / gradients for up to cap_pix pixels (B*H*W)
+  // activation / gradient planes for up to cap_pix padded pixels (B * H * padded_width(W))
   long long cap_pix = 0;
-  uint16_t* d_act[kLayers] = {};  // [0]: input (16 ch), [k]: output of layer k (32 ch), k = 1..7
-  uint16_t *d_g0 = nullptr, *d_g1 = nullptr;  // ping-pong gradients (32 ch)
+  uint4* d_act[kLayers] = {};  // [0]: input (16 ch), [k]: output of layer k (32 ch), k = 1..7
+  uint4 *d_g0 = nullptr, *d_g1 = nullptr;  // ping-pong gradients (32 ch)
+  uint4* d_zero = nullptr;     // kHalo zero chunks: the rows above and below an image
   float* d_loss = nullptr;
   int* d_err = nullptr;
   long long step = 0;
@@ -871,6 +884,7 @@ void cnn_destroy(hr_cnn* n) {
   }
   cudaFree(n->d_loss);
   cudaFree(n->d_err);
+  cudaFree(n->d_zero);
   delete n;
 }
 
@@ -893,11 +907,27 @@ int refresh_images(hr_cnn* n, cudaStream_t s) {
   return HR_OK;
 }
 
+// A caller's NHWC input into the planes d_act[0].
+int load_input(hr_cnn* n, const uint16_t* d_x, int B, int H, int W, cudaStream_t s) {
+  const long long rows = (long long)B * H;
+  const int Wp = padded_width(W);
+  HR_TRY(ensure_acts(n, rows * Wp));
+  const long long blocks = std::min<long long>((rows * Wp + 255) / 256, 16LL * hr::sm_count());
+  if (((uintptr_t)d_x & 15) == 0)
+    nhwc_to_planes_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
+  else
+    nhwc_to_planes_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
+  HR_CUDA_TRY(cudaGetLastError());
+  return HR_OK;
+}
+
 ConvArgs base_args(const hr_cnn* n, int B, int H, int W) {
   ConvArgs a{};
   a.B = B;
   a.H = H;
   a.W = W;
+  a.Wp = padded_width(W);
+  a.zero = n->d_zero;
   a.err = n->d_err;
   a.stall_row = n->stall_row;
   a.wait_limit = n->wait_limit;
@@ -955,6 +985,8 @@ extern "C" int hr_cnn_create(hr_cnn** net, const float* h_params) {
   }
   if (e == cudaSuccess) e = cudaMalloc(&n->d_loss, sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&n->d_err, sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc(&n->d_zero, kBox);
+  if (e == cudaSuccess) e = cudaMemset(n->d_zero, 0, kBox);
   if (e == cudaSuccess) e = cudaMemcpy(n->d_p, h_params, off * sizeof(float), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(n->d_m, 0, off * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(n->d_v, 0, off * sizeof(float));
@@ -996,8 +1028,7 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
   HR_REQUIRE(((uintptr_t)d_x & 15) == 0, "hr_cnn_train_step: input must be 16-byte aligned");
   cudaStream_t s = hr::as_stream(stream);
   const long long pix = (long long)B * H * W;
-  HR_TRY(ensure_acts(n, pix));
-  HR_CUDA_TRY(cudaMemcpyAsync(n->d_act[0], d_x, (size_t)pix * 16 * 2, cudaMemcpyDeviceToDevice, s));
+  HR_TRY(load_input(n, d_x, B, H, W, s));
   HR_CUDA_TRY(cudaMemsetAsync(n->d_loss, 0, sizeof(float), s));
   HR_CUDA_TRY(cudaMemsetAsync(n->d_g, 0, n->nparam * sizeof(float), s));
   HR_TRY(forward_trunk(n, B, H, W, s));
@@ -1016,18 +1047,18 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
   a.loss = n->d_loss;
   HR_TRY((launch_conv<32, 16, EPI_LOSS>(a, s)));
   // backward: G_k (gradient at layer k's output) -> dW_k, and G_{k-1} masked by act_{k-1} > 0
-  uint16_t* g = n->d_g0;
-  uint16_t* gn = n->d_g1;
+  uint4* g = n->d_g0;
+  uint4* gn = n->d_g1;
   for (int l = kLayers - 1; l >= 0; --l) {
     const int ci = kCin[l], co = kCout[l];
     float* dW = n->d_g + n->woff[l];
     float* db = n->d_g + n->boff[l];
     if (ci == 16)
-      HR_TRY((launch_wgrad<16, 32>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
+      HR_TRY((launch_wgrad<16, 32>(n->d_act[l], g, n->d_zero, B, H, W, dW, db, n->d_err, s)));
     else if (co == 16)
-      HR_TRY((launch_wgrad<32, 16>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
+      HR_TRY((launch_wgrad<32, 16>(n->d_act[l], g, n->d_zero, B, H, W, dW, db, n->d_err, s)));
     else
-      HR_TRY((launch_wgrad<32, 32>(n->d_act[l], g, B, H, W, dW, db, n->d_err, s)));
+      HR_TRY((launch_wgrad<32, 32>(n->d_act[l], g, n->d_zero, B, H, W, dW, db, n->d_err, s)));
     if (l == 0) break;
     ConvArgs b = base_args(n, B, H, W);
     b.in = g;
@@ -1057,17 +1088,9 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
   return HR_OK;
 }
 
-// Inference: out[b][y][x] = base + mu_w * net(x) for a batch of network inputs
-// (the same layouts as hr_cnn_train_step; base and out may use any strides).
-extern "C" int hr_cnn_forward(hr_cnn* n, float* d_out, const uint16_t* d_x, const float* d_base, long long sb,
-                              long long sp, int B, int H, int W, float mu_w, void* stream) {
-  HR_REQUIRE(n != nullptr && d_out != nullptr && d_x != nullptr && d_base != nullptr, "hr_cnn_forward: NULL argument");
-  HR_REQUIRE(B > 0 && H > 0 && W > 0 && mu_w > 0.0f, "hr_cnn_forward: invalid sizes");
-  cudaStream_t s = hr::as_stream(stream);
-  const long long pix = (long long)B * H * W;
-  HR_TRY(ensure_acts(n, pix));
-  if (d_x != n->d_act[0])
-    HR_CUDA_TRY(cudaMemcpyAsync(n->d_act[0], d_x, (size_t)pix * 16 * 2, cudaMemcpyDeviceToDevice, s));
+// Layers 1..8 from the input planes in d_act[0], with the residual epilogue.
+static int forward_residual(hr_cnn* n, float* d_out, const float* d_base, long long sb, long long sp, int B, int H,
+                            int W, float mu_w, cudaStream_t s) {
   HR_TRY(forward_trunk(n, B, H, W, s));
   ConvArgs a = base_args(n, B, H, W);
   a.in = n->d_act[7];
@@ -1081,6 +1104,17 @@ extern "C" int hr_cnn_forward(hr_cnn* n, float* d_out, const uint16_t* d_x, cons
   return launch_conv<32, 16, EPI_RESID>(a, s);
 }
 
+// Inference: out[b][y][x] = base + mu_w * net(x) for a batch of network inputs
+// (the same layouts as hr_cnn_train_step; base and out may use any strides).
+extern "C" int hr_cnn_forward(hr_cnn* n, float* d_out, const uint16_t* d_x, const float* d_base, long long sb,
+                              long long sp, int B, int H, int W, float mu_w, void* stream) {
+  HR_REQUIRE(n != nullptr && d_out != nullptr && d_x != nullptr && d_base != nullptr, "hr_cnn_forward: NULL argument");
+  HR_REQUIRE(B > 0 && H > 0 && W > 0 && mu_w > 0.0f, "hr_cnn_forward: invalid sizes");
+  cudaStream_t s = hr::as_stream(stream);
+  HR_TRY(load_input(n, d_x, B, H, W, s));
+  return forward_residual(n, d_out, d_base, sb, sp, B, H, W, mu_w, s);
+}
+
 // Corrects a whole reconstructed volume [YN][XN][ZN] (z fastest): every slice
 // with its two neighbours on each side (clamped at the ends), chunk slices at
 // a time. d_out must not alias d_vol.
@@ -1090,12 +1124,15 @@ extern "C" int hr_cnn_apply_volume(hr_cnn* n, float* d_out, const float* d_vol, 
   HR_REQUIRE((const void*)d_out != (const void*)d_vol, "hr_cnn_apply_volume: in-place correction is not supported");
   HR_REQUIRE(XN > 0 && YN > 0 && ZN > 0 && chunk > 0 && mu_w > 0.0f, "hr_cnn_apply_volume: invalid sizes");
   cudaStream_t s = hr::as_stream(stream);
-  HR_TRY(ensure_acts(n, (long long)std::min(chunk, ZN) * XN * YN));
+  const int Wp = padded_width(XN);
+  HR_TRY(ensure_acts(n, (long long)std::min(chunk, ZN) * YN * Wp));
   for (int z0 = 0; z0 < ZN; z0 += chunk) {
     const int nz = std::min(chunk, ZN - z0);
-    pack_input_kernel<<<8 * hr::sm_count(), 256, 0, s>>>(n->d_act[0], d_vol, XN, YN, ZN, z0, nz, 1.0f / mu_w);
+    HR_REQUIRE(YN <= 65535 && (nz + kPackZ - 1) / kPackZ <= 65535, "hr_cnn_apply_volume: grid too large");
+    const dim3 grid((Wp + kPackPx - 1) / kPackPx, YN, (nz + kPackZ - 1) / kPackZ);
+    pack_planes_kernel<<<grid, 256, 0, s>>>(n->d_act[0], d_vol, XN, YN, ZN, z0, nz, 1.0f / mu_w, Wp);
     HR_CUDA_TRY(cudaGetLastError());
-    HR_TRY(hr_cnn_forward(n, d_out + z0, n->d_act[0], d_vol + z0, 1, ZN, nz, YN, XN, mu_w, stream));
+    HR_TRY(forward_residual(n, d_out + z0, d_vol + z0, 1, ZN, nz, YN, XN, mu_w, s));
   }
   return HR_OK;
 }

@@ -47,3 +47,33 @@ def test_weight_gradients_vs_oracle(cuda, B, H, W):
             else:  # taps that reach no pixel (a one-pixel image), or next to none
                 assert np.linalg.norm(w[:, tap] - rw[:, tap]) < 3e-2 * np.linalg.norm(rw)
         o += n + co
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (2, 3, 127), (1, 5, 128), (2, 4, 129), (1, 2, 257)])
+def test_forward_after_other_shapes(cuda, B, H, W):
+    """Ragged widths around the 128-pixel tiles, after a run on a larger image
+    whose rows the buffers still hold, from an input that is not 16-byte
+    aligned: the same bits as a fresh network on an aligned input, which
+    matches the oracle (residual within 1e-3, BF16 storage on both sides)."""
+    rng = np.random.default_rng(W)
+    params = C.init_params(W, zero_last=False)
+    u = np.zeros((B, H, W, 16), dtype=np.float32)
+    u[..., :5] = rng.standard_normal((B, H, W, 5)).astype(np.float32) * 0.3
+    base = (MU_WATER * (1.0 + rng.standard_normal((B, H, W)) * 0.05)).astype(np.float32)
+    x = torch.from_numpy(u).to(torch.bfloat16).view(torch.int16).to(cuda)
+    tb = torch.from_numpy(base).to(cuda)
+    fresh = L.Corrector(params)
+    ref = fresh.forward(x, tb)
+    used = L.Corrector(params)
+    used.forward(torch.full((2, 9, 300, 16), 0x3f80, dtype=torch.int16, device=cuda),
+                 torch.ones((2, 9, 300), device=cuda))
+    shifted = torch.empty(x.numel() + 1, dtype=torch.int16, device=cuda)[1:]
+    shifted.copy_(x.reshape(-1))
+    assert shifted.data_ptr() % 16 == 2
+    got = used.forward(shifted.view(x.shape), tb)
+    for net in (fresh, used):
+        net.check()
+        net.close()
+    assert torch.equal(got, ref)
+    opred, _, _ = C.forward(params, C.bf16(u), base, MU_WATER)
+    assert rel_l2(ref.cpu().numpy() - base, opred - base) < 1e-3
