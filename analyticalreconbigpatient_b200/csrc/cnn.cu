@@ -18,17 +18,28 @@
 //
 // Convolutions run as implicit GEMMs on the 5th-generation tensor cores: one
 // tile is 128 output pixels of one image row (M = 128, TMEM lanes) by COUT
-// channels (N), K = 9 taps x CIN channels. The input rows lie in shared memory
+// channels, K = 9 taps x CIN channels. The input rows lie in shared memory
 // in the K-major no-swizzle layout (one plane of 16-byte pixel chunks per
-// 8-channel group), so the A operand of tap (dy, dx) is the same buffer seen
-// from another 16-byte-aligned start address: nine descriptor offsets replace
-// an im2col copy. The weights (B operand) stay in shared memory for the CTA's
-// life. Persistent, warp-specialised CTAs: warp 0 issues the copies into a
-// ring of input rows, warp 1 issues the 9*CIN/16 tcgen05.mma of a tile into
-// one of two TMEM accumulators, warps 2-5 read the other accumulator and run
-// the epilogue (bias + ReLU + BF16 store; gradient masking by the forward
+// 8-channel group), so the A operand of horizontal tap dx is the same buffer
+// seen 16 dx bytes further on: descriptor offsets replace an im2col copy.
+//
+// With N = COUT = 32 an MMA would spend its time reading A: 4 KB of shared
+// memory (32 clocks) for 16 clocks of multiplication, nine times per input
+// row. So the three vertical taps are stacked along N: input row r times the
+// weights of dy = 2, 1, 0 adds to output rows r - 1, r, r + 1, whose
+// accumulators are neighbouring column groups of a ring of kSlots in TMEM
+// (N = 96: one MMA per horizontal tap and 16 channels, 6 instead of 18 per
+// row, split in two where the three groups cross the ring's end). An output
+// row's sums run over (dy, dx, channels) in the same order as nine separate
+// taps', so the results are the same bits. 32 slices of 512 x 512, a 32 -> 32
+// layer: 267 -> 189 us (its bytes at the copy rate: 165 us).
+//
+// The weights (B operand) stay in shared memory for the CTA's life.
+// Persistent, warp-specialised CTAs: warp 0 issues the copies into a ring of
+// input rows, warp 1 the MMAs, warps 2-5 read the finished accumulators and
+// run the epilogue (bias + ReLU + BF16 store; gradient masking by the forward
 // activation; fused residual + loss + output gradient), so loads, MMAs and
-// stores of consecutive tiles overlap. Every mbarrier wait is bounded and sets
+// stores of consecutive rows overlap. Every mbarrier wait is bounded and sets
 // an error flag when it gives up. The backward data pass is the same kernel
 // with the weights transposed and flipped. Weight gradients are a second
 // tensor-core kernel that contracts over the pixels (wgrad_tc_kernel).
@@ -47,15 +58,22 @@ constexpr int kTileM = 128;                  // output pixels per tile (one row 
 constexpr int kHalo = kTileM + 2;            // halo pixels per row
 constexpr int kBox = kHalo * 16;             // bytes of one halo row: 130 pixel chunks of 8 channels
 constexpr int kPlane = 17 * 128;             // plane stride: one halo row, 128-byte aligned
-constexpr int kRing = 6;                     // halo ring: input rows in flight
+// Four CTAs per SM (the most that TMEM holds with four accumulators each) with a short ring: the epilogue's
+// latency per row, not the copies in flight, is what more CTAs hide (per 32 -> 32 layer of 32 slices of
+// 512 x 512: two CTAs with rings of 6 232 us, three 202, four with rings of 4 201, of 3 189).
+constexpr int kRing = 3;                     // halo ring: input rows in flight
+constexpr int kConvCtas = 4;                 // CTAs per SM that registers must allow
 constexpr int kThreads = 192;                // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
-constexpr int kTmemCols = 64;                // two 32-column accumulators
+constexpr int kSlots = 4;                    // accumulators in flight: three being added to, one being read
+// TMEM columns of a CTA. (More than it needs would be worse than a waste: the CTAs that registers and shared
+// memory let onto an SM wait there for TMEM while other SMs are idle.)
+constexpr int tmem_cols(int cout) { return kSlots * cout; }
 constexpr uint32_t kWaitLimit = 1u << 22;    // try_wait rounds before a wait is declared hung
 constexpr int kLayers = 8;
 constexpr int kCin[kLayers] = {16, 32, 32, 32, 32, 32, 32, 32};
 constexpr int kCout[kLayers] = {32, 32, 32, 32, 32, 32, 32, 16};
 
-enum Epi { EPI_RELU = 0, EPI_MASK = 1, EPI_LOSS = 2, EPI_RESID = 3 };
+enum Epi { EPI_RELU = 0, EPI_MASK = 1, EPI_LOSS = 2, EPI_RESID = 3, EPI_RAW = 4 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -159,8 +177,10 @@ __device__ __forceinline__ size_t plane_row(int b, int H, int y, int G, int c, i
 __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) |
-         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  uint32_t w;
+  memcpy(&w, &h, sizeof w);
+  return w;
 }
 
 template <int N>
@@ -192,23 +212,35 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float (&v)[32]) {
   }
 }
 
+// Zeros into N accumulator columns of the warp's 32 lanes.
+template <int N>
+__device__ __forceinline__ void tmem_zero(uint32_t taddr) {
+#pragma unroll
+  for (int c = 0; c < N; c += 16)
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+        "%1};" ::"r"(taddr + c),
+        "r"(0)
+        : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 struct ConvArgs {
   const uint4* in;       // input planes, CIN / 8 groups
   const uint4* zero;     // kHalo zero chunks
-  const uint16_t* wimg;  // B operand image [9*CIN/8][COUT][8] BF16
+  const uint16_t* wimg;  // B operand image [3*CIN/8][3*COUT][8] BF16
   const float* bias;     // [COUT] (EPI_RELU, EPI_LOSS, EPI_RESID)
   uint4* out;            // output planes, COUT / 8 groups (EPI_RELU, EPI_MASK); output gradient (EPI_LOSS)
   const uint4* mask;     // planes of the forward activation whose > 0 passes the gradient (EPI_MASK)
   // residual epilogues: element (b, y, x) of base/target/pred at b*sb + (y*W + x)*sp
   const float* base;
   const float* target;   // EPI_LOSS
-  float* pred;           // EPI_RESID output (EPI_LOSS: optional)
+  float* pred;           // EPI_RESID output (EPI_LOSS: optional); EPI_RAW: channel 0 itself, [B][H][W]
   long long sb, sp;
   float scale;           // mu_w: pred = base + scale * r
   float grad_scale;      // EPI_LOSS: d loss / d r = grad_scale * (pred - target) / scale
   float* loss;           // EPI_LOSS: accumulates sum ((pred - target) / scale)^2
   int B, H, W, Wp;
-  int rows_per_unit;     // output rows a CTA computes down one 128-pixel column strip
   int* err;
   int stall_row;         // test hook: the CTA's input row of this index is never loaded (-1: none)
   uint32_t wait_limit;   // polls before a pipeline wait gives up
@@ -221,7 +253,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
   const bool valid = x < a.W;  // pixels beyond the image are stored as zeros
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   const size_t row = plane_row(b, a.H, y, COUT / 8, 0, a.Wp);
-  if constexpr (EPI != EPI_RESID) {  // the zero chunks before the first and after the last tile pixel
+  if constexpr (EPI != EPI_RESID && EPI != EPI_RAW) {  // the zero chunks before the first and after the last tile pixel
     if (x == 0 || x == a.Wp - 3) {
 #pragma unroll
       for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + (x == 0 ? 0 : a.Wp - 1)] = zero;
@@ -231,9 +263,12 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
     uint4* o = a.out + row + x + 1;
 #pragma unroll
     for (int c = 0; c < COUT / 8; ++c) {
+      const float4* bp = reinterpret_cast<const float4*>(bias_s) + 2 * c;
+      const float4 b0 = bp[0], b1 = bp[1];
+      const float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
       float u[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = fmaxf(v[8 * c + j] + bias_s[8 * c + j], 0.0f);
+      for (int j = 0; j < 8; ++j) u[j] = fmaxf(v[8 * c + j] + bias[j], 0.0f);
       o[(size_t)c * a.Wp] = valid ? make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]),
                                                pack2(u[6], u[7]))
                                   : zero;
@@ -253,6 +288,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
       }
       o[(size_t)c * a.Wp] = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]), pack2(u[6], u[7]));
     }
+  } else if constexpr (EPI == EPI_RAW) {
+    if (valid) a.pred[((size_t)b * a.H + y) * a.W + x] = v[0] + bias_s[0];
   } else {
     const float r = v[0] + bias_s[0];
     float e2 = 0.0f;
@@ -280,12 +317,11 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
 }
 
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_constant__ ConvArgs a) {
+__global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __grid_constant__ ConvArgs a) {
   constexpr int G = CIN / 8;                 // 8-channel groups (copies per input row)
   constexpr int kRow = G * kPlane;           // bytes of one input row (130 pixels)
   constexpr int kWBytes = 9 * CIN * COUT * 2;
-  constexpr int kKSteps = 9 * CIN / 16;
-  constexpr uint32_t kIdesc = idesc_bf16(COUT);
+  constexpr int kKSteps = 3 * CIN / 16;      // per input row: horizontal taps x 16-channel steps
   constexpr uint32_t kTxBytes = G * kBox;
   static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "unsupported channel counts");
   extern __shared__ uint8_t smem_raw[];
@@ -294,8 +330,8 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
   uint64_t* full = reinterpret_cast<uint64_t*>(wsm + kWBytes);
   uint64_t* empty = full + kRing;
   uint64_t* tfull = empty + kRing;
-  uint64_t* tempty = tfull + 2;
-  uint64_t* mdone = tempty + 2;  // the MMA issuer's last commit (one spare slot keeps 16-byte alignment)
+  uint64_t* tempty = tfull + kSlots;
+  uint64_t* mdone = tempty + kSlots;  // the MMA issuer's last commit (one spare slot keeps 16-byte alignment)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* bias_s = reinterpret_cast<float*>(tmem_slot + 4);  // 16-byte aligned, COUT floats
@@ -310,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kSlots; ++s) {
       mbar_init(&tfull[s], 1);
       mbar_init(&tempty[s], 128);
     }
@@ -320,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kTmemCols));
+                 "r"(tmem_cols(COUT)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   __syncthreads();
@@ -328,24 +364,28 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
   const uint32_t tmem = *tmem_slot;
   const uint32_t smem_a = smem_u32(smem), w_a = smem_u32(wsm);
 
-  // Work units: (image b, 128-pixel column strip seg, chunk of rows_per_unit output rows). Down a
-  // strip each input row is loaded once into the ring and serves three consecutive output rows;
-  // a unit of n output rows loads n + 2 input rows (zero rows above and below the image).
+  // The B x H output rows are cut into equal shares of consecutive rows, one per group of nseg CTAs, and
+  // each CTA of a group takes one 128-pixel column strip of the share: every CTA has the same work to
+  // within a row (chunks of fixed length left five rounds of work for 4.1 rounds' worth at 8 images), and
+  // a group's copies and stores fall into the same stretch of memory at about the same time (with every
+  // CTA on a stretch of its own a 32 -> 32 layer of 32 slices of 512 x 512 took 248 us, so 202). A share
+  // crosses from one image to the next in pieces; a piece of n output rows loads n + 2 input rows (zero
+  // rows above and below the image).
   const int nseg = (a.W + kTileM - 1) / kTileM;
-  const int rpu = a.rows_per_unit;
-  const int nchunk = (a.H + rpu - 1) / rpu;
-  const long long units = (long long)a.B * nseg * nchunk;
+  const int seg = blockIdx.x % nseg, groups = gridDim.x / nseg, group = blockIdx.x / nseg;
+  const long long rows = (long long)a.B * a.H;
+  const long long r0 = rows * group / groups, r1 = rows * (group + 1) / groups;
   if (warp == 0) {
-    // ---- producer: input rows of each unit into the ring, G halo rows each -------------------
+    // ---- producer: input rows of each piece into the ring, G halo rows each ------------------
     if (lane == 0) {
       int h = 0;  // input rows loaded by this CTA
       int last_h[kRing];
       for (int s = 0; s < kRing; ++s) last_h[s] = -1;
       bool ok = true;
-      for (long long un = blockIdx.x; un < units && ok; un += gridDim.x) {
-        const int seg = (int)(un % nseg), chunk = (int)((un / nseg) % nchunk);
-        const int b = (int)(un / ((long long)nseg * nchunk));
-        const int y0 = chunk * rpu, ny = min(rpu, a.H - y0);
+      for (long long r = r0; r < r1 && ok;) {
+        const int b = (int)(r / a.H);
+        const int y0 = (int)(r - (long long)b * a.H), ny = (int)min((long long)(a.H - y0), r1 - r);
+        r += ny;
         for (int j = 0; j < ny + 2; ++j, ++h) {
           const int s = h % kRing;
           if (h >= kRing && !mbar_wait(&empty[s], ((h / kRing) - 1) & 1, abort_flag, a.err, a.wait_limit)) {
@@ -367,40 +407,39 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
         if (last_h[s] >= 0) mbar_drain(&full[s], (last_h[s] / kRing) & 1, a.err, a.wait_limit);
     }
   } else if (warp == 1) {
-    // ---- MMA issuer: output row i of a unit reads input rows i, i+1, i+2 of the unit ---------
+    // ---- MMA issuer: input row i of a piece adds to its output rows i - 2, i - 1 and i -------
     if (lane == 0) {
-      int hbase = 0, o = 0;
+      int h = 0, obase = 0;  // input rows consumed; output rows of the pieces before
       bool ok = true;
-      for (long long un = blockIdx.x; un < units && ok; un += gridDim.x) {
-        const int chunk = (int)((un / nseg) % nchunk);
-        const int ny = min(rpu, a.H - chunk * rpu);
-        for (int i = 0; i < ny && ok; ++i, ++o) {
-          for (int j = (i == 0 ? 0 : 2); j < 3 && ok; ++j) {
-            const int hh = hbase + i + j;
-            ok = mbar_wait(&full[hh % kRing], (hh / kRing) & 1, abort_flag, a.err, a.wait_limit);
-          }
-          const int acc = o & 1;
-          if (ok && o >= 2) ok = mbar_wait(&tempty[acc], ((o >> 1) - 1) & 1, abort_flag, a.err, a.wait_limit);
+      for (long long r = r0; r < r1 && ok;) {
+        const int ny = (int)min((long long)(a.H - (int)(r % a.H)), r1 - r);
+        r += ny;
+        for (int i = 0; i < ny + 2; ++i, ++h) {
+          const int s = h % kRing;
+          ok = mbar_wait(&full[s], (h / kRing) & 1, abort_flag, a.err, a.wait_limit);
+          const int o = obase + i;  // the output row that starts here (if i < ny)
+          if (ok && i < ny) ok = mbar_wait(&tempty[o % kSlots], (o / kSlots) & 1, abort_flag, a.err, a.wait_limit);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const int lo = max(i - 2, 0), hi = min(i, ny - 1);  // output rows of the piece
+          const int first = (obase + lo) % kSlots, n = hi - lo + 1, m = min(n, kSlots - first);
+          // the n column groups from row lo's on, in two where they cross the end of the ring; weights of
+          // dy = i - lo downwards
+          const uint32_t d0 = tmem + (uint32_t)first * COUT;
+          const uint32_t bw = w_a + (uint32_t)(2 - (i - lo)) * (COUT * 16);
+          const uint32_t id0 = idesc_bf16(m * COUT), id1 = idesc_bf16((n - m) * COUT);
 #pragma unroll
           for (int k = 0; k < kKSteps; ++k) {
-            const int k0 = k * 16;
-            const int tap = k0 / CIN, c0 = k0 - tap * CIN;
-            const int dy = tap / 3, dx = tap - dy * 3;  // input row and pixel offset
-            const uint32_t row = smem_a + ((hbase + i + dy) % kRing) * kRow;
-            const uint64_t ad = desc_noswz(row + (c0 / 8) * kPlane + dx * 16, kPlane, 128);
-            const uint64_t bd = desc_noswz(w_a + (k0 / 8) * (COUT * 16), COUT * 16, 128);
-            umma(tmem + acc * 32, ad, bd, kIdesc, k > 0 ? 1u : 0u);
+            const int dx = k / (CIN / 16), c0 = (k - dx * (CIN / 16)) * 16;
+            const uint64_t ad = desc_noswz(smem_a + s * kRow + (c0 / 8) * kPlane + dx * 16, kPlane, 128);
+            const uint32_t b = bw + (uint32_t)(dx * G + c0 / 8) * (3 * COUT * 16);
+            umma(d0, ad, desc_noswz(b, 3 * COUT * 16, 128), id0, 1u);
+            if (m < n) umma(tmem, ad, desc_noswz(b + (uint32_t)m * (COUT * 16), 3 * COUT * 16, 128), id1, 1u);
           }
-          umma_commit(&tfull[acc]);                       // the accumulator is ready
-          umma_commit(&empty[(hbase + i) % kRing]);        // input row i serves no later output row
-          if (i == ny - 1) {
-            umma_commit(&empty[(hbase + i + 1) % kRing]);  // the unit's last two input rows
-            umma_commit(&empty[(hbase + i + 2) % kRing]);
-          }
+          umma_commit(&empty[s]);                                    // the input row has been read
+          if (i >= 2) umma_commit(&tfull[(obase + i - 2) % kSlots]);  // output row i - 2 is complete
         }
-        hbase += ny + 2;
+        obase += ny;
       }
       // every tensor-core operation issued above completes before TMEM is freed
       umma_commit(mdone);
@@ -408,24 +447,30 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
     }
   } else {
     // ---- epilogue: warps 2-5, TMEM lane quarter warp % 4 --------------------------------------
+    // Every accumulator is handed to the MMAs as zeros, so that one instruction may add to three.
     const int q = warp & 3;
+    const uint32_t quarter = tmem + ((uint32_t)(q * 32) << 16);
+    tmem_zero<COUT * kSlots>(quarter);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    for (int s = 0; s < kSlots; ++s) mbar_arrive(&tempty[s]);
     int it = 0;
     bool ok = true;
-    for (long long un = blockIdx.x; un < units && ok; un += gridDim.x) {
-      const int seg = (int)(un % nseg), chunk = (int)((un / nseg) % nchunk);
-      const int b = (int)(un / ((long long)nseg * nchunk));
-      const int y0 = chunk * rpu, ny = min(rpu, a.H - y0);
+    for (long long r = r0; r < r1 && ok;) {
+      const int b = (int)(r / a.H);
+      const int y0 = (int)(r - (long long)b * a.H), ny = (int)min((long long)(a.H - y0), r1 - r);
+      r += ny;
       for (int i = 0; i < ny; ++i, ++it) {
-        const int acc = it & 1;
-        if (!mbar_wait(&tfull[acc], (it >> 1) & 1, abort_flag, a.err, a.wait_limit)) {
+        const int acc = it % kSlots;
+        if (!mbar_wait(&tfull[acc], (it / kSlots) & 1, abort_flag, a.err, a.wait_limit)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         float v[COUT];
-        tmem_ld<COUT>(tmem + acc * 32 + ((uint32_t)(q * 32) << 16), v);
+        tmem_ld<COUT>(quarter + acc * COUT, v);
+        tmem_zero<COUT>(quarter + acc * COUT);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&tempty[acc]);  // the registers hold the tile: the accumulator may be reused
+        mbar_arrive(&tempty[acc]);  // the registers hold the row: the accumulator may be reused
         conv_epilogue<COUT, EPI>(a, v, bias_s, b, y0 + i, seg * kTileM + q * 32 + lane, lane);
       }
     }
@@ -433,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, 3) conv_tc_kernel(const __grid_const
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(COUT)));
   }
 }
 
@@ -674,19 +719,20 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
 }
 
 // Master FP32 weights W[co][tap][ci] -> BF16 operand images:
-//   forward  B[n = co][k = tap*CIN + ci]             at [(k/8)][co][k%8]
-//   backward B[n = ci][k = tap'*COUT + co] = W[co][8 - tap'][ci]  at [(k/8)][ci][k%8]
+//   forward  B[n = (2 - dy)*COUT + co][k = dx*CIN + ci]  at [(k/8)][n][k%8]  (tap = 3 dy + dx)
+//   backward the same with channels exchanged and taps reversed: tap' = 8 - tap, n = (2 - dy')*CIN + ci,
+//            k = dx'*COUT + co
 __global__ void weight_images_kernel(const float* __restrict__ w, uint16_t* __restrict__ fwd,
                                      uint16_t* __restrict__ bwd, int CIN, int COUT) {
   const int n = 9 * CIN * COUT;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int ci = i % CIN, tap = (i / CIN) % 9, co = i / (9 * CIN);
     const uint16_t v = __bfloat16_as_ushort(__float2bfloat16_rn(w[i]));
-    const int kf = tap * CIN + ci;
-    fwd[((size_t)(kf / 8) * COUT + co) * 8 + kf % 8] = v;
+    const int kf = tap % 3 * CIN + ci, nf = (2 - tap / 3) * COUT + co;
+    fwd[((size_t)(kf / 8) * 3 * COUT + nf) * 8 + kf % 8] = v;
     if (bwd) {
-      const int kb = (8 - tap) * COUT + co;
-      bwd[((size_t)(kb / 8) * CIN + ci) * 8 + kb % 8] = v;
+      const int kb = (2 - tap % 3) * COUT + co, nb = tap / 3 * CIN + ci;  // dy' = 2 - dy, dx' = 2 - dx
+      bwd[((size_t)(kb / 8) * 3 * CIN + nb) * 8 + kb % 8] = v;
     }
   }
 }
@@ -761,6 +807,28 @@ __global__ void __launch_bounds__(256) pack_planes_kernel(uint4* __restrict__ ou
   }
 }
 
+// The residual epilogue of a whole volume: out = vol + scale r for slices [z0, z0 + nz), r by slices
+// ([nz][YN][XN]), the volume with z fastest. A CTA turns 32 pixels x 32 slices through shared memory, so that
+// both sides are read and written in runs. (From the convolution's epilogue, slice by slice, every 4-byte
+// access of the volume was a sector of its own: that layer took 272 us per 32 slices of 512 x 512, now 119
+// with this kernel's 37.)
+__global__ void __launch_bounds__(256) add_residual_kernel(float* __restrict__ out, const float* __restrict__ vol,
+                                                           const float* __restrict__ r, long long px, int ZN, int z0,
+                                                           int nz, float scale) {
+  __shared__ float t[32][33];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const long long p0 = (long long)blockIdx.x * 32;
+  const int s0 = blockIdx.y * 32;
+  for (int k = row; k < 32; k += 8)
+    if (s0 + k < nz && p0 + lane < px) t[k][lane] = r[(size_t)(s0 + k) * px + p0 + lane];
+  __syncthreads();
+  for (int p = row; p < 32; p += 8)
+    if (s0 + lane < nz && p0 + p < px) {
+      const size_t o = (size_t)(p0 + p) * ZN + z0 + s0 + lane;
+      out[o] = vol[o] + scale * t[lane][p];
+    }
+}
+
 // A caller's NHWC input [rows][W][16] as planes (ALIGNED: it starts on a 16-byte boundary).
 template <bool ALIGNED>
 __global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* __restrict__ in, long long rows, int W,
@@ -789,7 +857,7 @@ __global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* _
 // Dynamic shared memory of a conv CTA: input-row ring + weights + barriers + alignment slack.
 template <int CIN, int COUT>
 constexpr size_t conv_smem() {
-  return (size_t)kRing * (CIN / 8) * kPlane + 9 * CIN * COUT * 2 + 256 + COUT * 4 + 128;  // barriers fit in 256
+  return (size_t)kRing * (CIN / 8) * kPlane + 9 * CIN * COUT * 2 + 512 + COUT * 4 + 128;  // barriers fit in 512
 }
 
 template <int CIN, int COUT, int EPI>
@@ -809,15 +877,14 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
   HR_CUDA_TRY(cudaGetDevice(&dev));
   HR_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   const int by_smem = smem_sm / (int)(smem + fa.sharedSizeBytes + 1024);
-  const int by_tmem = 512 / kTmemCols;
+  const int by_tmem = 512 / tmem_cols(COUT);
   const int by_regs = 65536 / std::max(1, fa.numRegs * kThreads);
   const int per_sm = std::max(1, std::min({by_smem, by_tmem, by_regs, 2048 / kThreads}));
   const long long ctas = (long long)per_sm * hr::sm_count();
-  // rows per unit: about four units per resident CTA (balance), at least 4 rows (each unit reloads 2 rows)
-  const long long strips = (long long)a.B * ((a.W + kTileM - 1) / kTileM);
-  a.rows_per_unit = (int)std::min<long long>(64, std::max<long long>(4, strips * a.H / (4 * ctas)));
-  const long long units = strips * ((a.H + a.rows_per_unit - 1) / a.rows_per_unit);
-  const long long grid = std::min<long long>(units, ctas);
+  // one share of the rows per group of CTAs that fit together, of at least 4 rows (each reloads 2 rows)
+  const long long nseg = (a.W + kTileM - 1) / kTileM;
+  const long long groups = std::min(((long long)a.B * a.H + 3) / 4, std::max(1LL, ctas / nseg));
+  const long long grid = groups * nseg;
   if (grid <= 0) return HR_OK;
   conv_tc_kernel<CIN, COUT, EPI><<<(unsigned)grid, kThreads, smem, s>>>(a);
   HR_CUDA_TRY(cudaGetLastError());
@@ -1132,7 +1199,17 @@ extern "C" int hr_cnn_apply_volume(hr_cnn* n, float* d_out, const float* d_vol, 
     const dim3 grid((Wp + kPackPx - 1) / kPackPx, YN, (nz + kPackZ - 1) / kPackZ);
     pack_planes_kernel<<<grid, 256, 0, s>>>(n->d_act[0], d_vol, XN, YN, ZN, z0, nz, 1.0f / mu_w, Wp);
     HR_CUDA_TRY(cudaGetLastError());
-    HR_TRY(forward_residual(n, d_out + z0, d_vol + z0, 1, ZN, nz, YN, XN, mu_w, s));
+    HR_TRY(forward_trunk(n, nz, YN, XN, s));
+    ConvArgs a = base_args(n, nz, YN, XN);
+    a.in = n->d_act[7];
+    a.wimg = n->d_wf[7];
+    a.bias = n->d_p + n->boff[7];
+    a.pred = reinterpret_cast<float*>(n->d_g0);  // free between training steps
+    HR_TRY((launch_conv<32, 16, EPI_RAW>(a, s)));
+    const long long px = (long long)XN * YN;
+    const dim3 rgrid((unsigned)((px + 31) / 32), (nz + 31) / 32);
+    add_residual_kernel<<<rgrid, 256, 0, s>>>(d_out, d_vol, a.pred, px, ZN, z0, nz, mu_w);
+    HR_CUDA_TRY(cudaGetLastError());
   }
   return HR_OK;
 }
