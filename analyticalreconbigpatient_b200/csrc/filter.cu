@@ -8,7 +8,8 @@
 // The reference computes a linear convolution f[j] = sum_m p[m] h[j-m] with
 // |j-m| <= YL-1 through a length-NN circular one. Any circular length
 // N >= 2 YL - 1 gives the same linear convolution, so this filter uses
-// N = 2^ceil(log2(2 YL - 1)) (2048 for YL = 888, the reference pads to 4096).
+// N = 2^ceil(log2(2 YL - 1)) (2048 for YL = 888, the reference pads to 4096),
+// raised to 2048 from 512 on.
 // h is even, so its transform H is real; two real rows a, b are filtered at
 // once as one complex signal a + i b:  ifft(H fft(a + i b)) = (h*a) + i (h*b).
 // The inverse transform is done with the forward one: ifft(Z) =
@@ -22,8 +23,8 @@
 // layout [v][ZL][YL] or in the rebinning's layout [v][YL][ZL]; for the latter
 // the 4 rows of a tile are 16 contiguous bytes per channel.
 //
-// N = 2048 (YL in (512, 1024], the scanners' 888 channels) runs a register-
-// resident kernel instead: one warp per pair of rows, 64 points per lane
+// N = 2048 (YL in (128, 1024], the scanners' 888 channels) runs a register-
+// resident kernel instead: two warps per pair of rows (below), or one, 64 points per lane
 // (N = 64 x 32). Forward: each lane j transforms x[j + 32 m] over m with a
 // 64-point DFT (8 x 8, in registers), multiplies by W_2048^(j c), and the
 // warp exchanges through shared memory so that lane t holds columns c = t,
@@ -569,14 +570,45 @@ int launch(const hr_filter_plan* p, float* out, const float* in, int view0, cuda
 //   A': lane j: inverse 32-point DFT over k1 of row j -> y[j + 64 m].
 // With YL <= 64 MNZ only m < MNZ carries samples (888 channels: 14 of 32), so
 // the first forward stage and the last inverse one are pruned at compile time.
+//
+// Sixteen warps per SM (128 registers) do not hide a DRAM latency at the head
+// of every pair, so the next pair's rows are asked into L2 while this one is
+// transformed and, where they are not staged through shared memory, loaded
+// into registers before this one's last DFT; one twiddle table for both uses
+// leaves L1 room for the preweights (a CTA meets the same rows k over and
+// over: the grid's stride is a multiple of common ZL). 1023 x 32 rows of 888:
+// 226 -> 151 us; staged (rebinning layout) 174 -> 152 us; 4000 x 64: 1657 ->
+// 1096 us (of which the L2 requests 311, registers 47, the table 203). The
+// same sums, so the same bits.
 // Bank-conflict free: rows of 33 float2 for the row-wise stages, 16
 // consecutive columns per half-warp for the column-wise one.
 constexpr int kPairs = 4;             // row pairs per CTA, two warps each
 constexpr int kThreads2 = 64 * kPairs;
 constexpr int kS2 = 33;               // exchange row stride in float2
+constexpr int kT2 = 65;               // twiddle row stride: read along j (A) and along k1 (B), both without conflicts
 
 __device__ __forceinline__ void bar_pair(int pair) {
   asm volatile("bar.sync %0, %1;" ::"r"(1 + pair), "r"(64) : "memory");
+}
+
+// Asks for the samples of the row pair (STAGE: the CTA's four pairs) from `pt` on to be brought into L2.
+template <int IN_LAYOUT, bool STAGE>
+__device__ __forceinline__ void prefetch_rows(const float* in, int YL, int ZL, long long rows, int view0,
+                                              long long pt) {
+  if constexpr (STAGE) {  // 32 bytes of every channel
+    const long long r0 = 2 * pt, v0 = r0 / ZL;
+    const float* src = in + (size_t)(view0 + v0) * YL * ZL + (r0 - v0 * ZL);
+    for (int t = threadIdx.x; t < YL; t += kThreads2)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(src + (size_t)t * ZL) : "memory");
+  } else if constexpr (IN_LAYOUT == HR_LAYOUT_ROWS) {  // two rows on end: the 16-byte blocks they hold
+    if ((threadIdx.x & 63) == 0) {
+      const float* src = in + (size_t)view0 * ZL * YL + (size_t)(2 * pt) * YL;
+      const uintptr_t lo = ((uintptr_t)src + 15) & ~(uintptr_t)15;
+      const uintptr_t hi = (uintptr_t)(src + (size_t)(rows - 2 * pt < 2 ? 1 : 2) * YL) & ~(uintptr_t)15;
+      if (hi > lo)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((uint32_t)(hi - lo)) : "memory");
+    }
+  }
 }
 
 template <int IN_LAYOUT, bool STAGE, int MNZ>
@@ -587,15 +619,10 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
                                                                    const float* __restrict__ wt, int YL, int ZL,
                                                                    long long rows, int view0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* twA = reinterpret_cast<float2*>(smem_raw);  // [32][64]: W_2048^(j k1) at [k1][j]
-  float2* twB = twA + 32 * 64;                        // [64][32]: the same at [j][k1]
-  float2* G = twB + 64 * 32;                          // [32][32]: {H0 + H1, H0 - H1} at [k][k1]
-  float2* xall = G + 32 * 32;                         // kPairs exchange buffers [64][kS2]
-  for (int t = threadIdx.x; t < 32 * 64; t += kThreads2) {
-    const float2 w = gtw[t];
-    twA[t] = w;
-    twB[(t & 63) * 32 + (t >> 6)] = w;
-  }
+  float2* tw = reinterpret_cast<float2*>(smem_raw);  // [32][kT2]: W_2048^(j k1) at [k1][j]
+  float2* G = tw + 32 * kT2;                         // [32][32]: {H0 + H1, H0 - H1} at [k][k1]
+  float2* xall = G + 32 * 32;                        // kPairs exchange buffers [64][kS2]
+  for (int t = threadIdx.x; t < 32 * 64; t += kThreads2) tw[(t >> 6) * kT2 + (t & 63)] = gtw[t];
   for (int t = threadIdx.x; t < 32 * 32; t += kThreads2) G[t] = gG[t];
   __syncthreads();
   const int pair = threadIdx.x >> 6, h = (threadIdx.x >> 5) & 1, lane = threadIdx.x & 31;
@@ -607,11 +634,34 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
   // STAGE: rows is a multiple of 8, so every tile of kPairs pairs is full and the loop is CTA-uniform
   const long long first = STAGE ? (long long)blockIdx.x * kPairs : (long long)blockIdx.x * kPairs + pair;
   const long long step = (long long)gridDim.x * kPairs;
+  [[maybe_unused]] float2 next[MNZ];  // the samples of the next pair of rows
+  [[maybe_unused]] auto fetch = [&](long long pr) {
+    const long long ra = 2 * pr, rb = ra + 1;
+    const int ka = (int)(ra % ZL), kb = (int)(rb % ZL);
+    const long long va = ra / ZL, vb = rb / ZL;
+    const float* pa = IN_LAYOUT == HR_LAYOUT_ROWS ? in + ((size_t)(view0 + va) * ZL + ka) * YL
+                                                  : in + (size_t)(view0 + va) * YL * ZL + ka;
+    const float* pb = IN_LAYOUT == HR_LAYOUT_ROWS ? in + ((size_t)(view0 + vb) * ZL + kb) * YL
+                                                  : in + (size_t)(view0 + vb) * YL * ZL + kb;
+    const size_t es = IN_LAYOUT == HR_LAYOUT_ROWS ? 1 : (size_t)ZL;  // element stride along a row
+#pragma unroll
+    for (int m = 0; m < MNZ; ++m) {
+      const int n = j + 64 * m;
+      next[m] = make_float2(0.0f, 0.0f);
+      if (n < YL) {
+        next[m].x = __ldg(pa + n * es);
+        if (rb < rows) next[m].y = __ldg(pb + n * es);
+      }
+    }
+  };
+  if constexpr (!STAGE)
+    if (first < npairs) fetch(first);
   for (long long pt = first; pt < npairs; pt += step) {
     const long long pr = STAGE ? pt + pair : pt;
     const long long ra = 2 * pr, rb = ra + 1;
     const bool hasb = rb < rows;
     float2 v[32];
+    if (pt + step < npairs) prefetch_rows<IN_LAYOUT, STAGE>(in, YL, ZL, rows, view0, pt + step);
     if constexpr (STAGE) {
       // rows 2 pt .. 2 pt + 7 are k0 .. k0 + 7 of one view (ZL % 8 == 0): stage them preweighted
       const long long r0 = 2 * pt;
@@ -639,24 +689,13 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
       __syncthreads();  // the staging area is read before any pair writes its exchange buffer
     } else {
       bar_pair(pair);  // both warps of the pair have finished reading the buffer (the previous pair of rows)
-      const int ka = (int)(ra % ZL), kb = (int)(rb % ZL);
-      const long long va = ra / ZL, vb = rb / ZL;
-      const float* pa = IN_LAYOUT == HR_LAYOUT_ROWS ? in + ((size_t)(view0 + va) * ZL + ka) * YL
-                                                    : in + (size_t)(view0 + va) * YL * ZL + ka;
-      const float* pb = IN_LAYOUT == HR_LAYOUT_ROWS ? in + ((size_t)(view0 + vb) * ZL + kb) * YL
-                                                    : in + (size_t)(view0 + vb) * YL * ZL + kb;
-      const size_t es = IN_LAYOUT == HR_LAYOUT_ROWS ? 1 : (size_t)ZL;  // element stride along a row
-      const float* wa = wt + (size_t)ka * YL;
-      const float* wb = wt + (size_t)kb * YL;
+      const float* wa = wt + (size_t)(ra % ZL) * YL;
+      const float* wb = wt + (size_t)(rb % ZL) * YL;
 #pragma unroll
       for (int m = 0; m < 32; ++m) {
         const int n = j + 64 * m;
-        float a = 0.0f, b = 0.0f;
-        if (m < MNZ && n < YL) {
-          a = __ldg(pa + n * es) * __ldg(wa + n);
-          if (hasb) b = __ldg(pb + n * es) * __ldg(wb + n);
-        }
-        v[m] = make_float2(a, b);
+        v[m] = make_float2(0.0f, 0.0f);
+        if (m < MNZ && n < YL) v[m] = make_float2(next[m].x * __ldg(wa + n), next[m].y * __ldg(wb + n));
       }
     }
     // ---- A: 32-point DFT over m, twiddle, row j of the buffer --------------
@@ -664,7 +703,7 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
 #pragma unroll
     for (int p = 0; p < 32; ++p) {
       const int k1 = dft32_freq(p);
-      xb[j * kS2 + k1] = cmulw<false>(v[p], twA[k1 * 64 + j]);
+      xb[j * kS2 + k1] = cmulw<false>(v[p], tw[k1 * kT2 + j]);
     }
     bar_pair(pair);
     // ---- B: column kc, rows of parity e: DFT over j', exchange + filter, inverse
@@ -686,12 +725,14 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
 #pragma unroll
     for (int q = 0; q < 32; ++q) {
       const int jj = 2 * q + e;
-      xb[jj * kS2 + kc] = cmulw<true>(v[q], twB[jj * 32 + kc]);
+      xb[jj * kS2 + kc] = cmulw<true>(v[q], tw[kc * kT2 + jj]);
     }
     bar_pair(pair);
     // ---- A': inverse 32-point DFT over k1 of row j: y[j + 64 m] -------------
 #pragma unroll
     for (int p = 0; p < 32; ++p) v[p] = xb[j * kS2 + dft32_freq(p)];
+    if constexpr (!STAGE)
+      if (pt + step < npairs) fetch(pt + step);
     dft32_inv(v);
     float* oa = out + (size_t)ra * YL;
     float* ob = out + (size_t)rb * YL;
@@ -706,7 +747,7 @@ __global__ void __launch_bounds__(kThreads2, 2) filter2048x2_kernel(float* __res
   }
 }
 
-size_t smem_bytes2() { return (2 * 32 * 64 + 32 * 32 + kPairs * 64 * kS2) * sizeof(float2); }
+size_t smem_bytes2() { return (32 * kT2 + 32 * 32 + kPairs * 64 * kS2) * sizeof(float2); }
 
 template <int IN_LAYOUT, bool STAGE, int MNZ>
 int launch_k2(const hr_filter_plan* p, float* out, const float* in, int view0, cudaStream_t s) {
@@ -728,6 +769,8 @@ int launch_k2(const hr_filter_plan* p, float* out, const float* in, int view0, c
 
 template <int IN_LAYOUT, bool STAGE>
 int launch_k2m(const hr_filter_plan* p, float* out, const float* in, int view0, cudaStream_t s) {
+  if (p->YL <= 64 * 8) return launch_k2<IN_LAYOUT, STAGE, 8>(p, out, in, view0, s);
+  if (p->YL <= 64 * 10) return launch_k2<IN_LAYOUT, STAGE, 10>(p, out, in, view0, s);
   if (p->YL <= 64 * 14) return launch_k2<IN_LAYOUT, STAGE, 14>(p, out, in, view0, s);
   return launch_k2<IN_LAYOUT, STAGE, 16>(p, out, in, view0, s);
 }
@@ -822,6 +865,11 @@ extern "C" int hr_filter_plan_create(hr_filter_plan** plan, int YL, int ZL, int 
   HR_TRY(hr::require_device());
   int log2N = 3;
   while ((1 << log2N) < 2 * YL - 1) ++log2N;
+  // Lengths 512 and 1024 run as 2048 too: the register kernel's longer transforms, pruned to the samples there
+  // are, cost less than the shared-memory kernel's short ones, and their results are nearer to FP64 (32,000
+  // rows of 500 channels 246 -> 126 us, error 5.1e-6 -> 4.4e-6; of 250 channels 138 -> 119 us, 3.1e-6 ->
+  // 2.4e-6; of 100 channels, N = 256, it would be 66 -> 116 us).
+  if (log2N == 9 || log2N == 10) log2N = 11;
   const int N = 1 << log2N;
   // Wrapped kernel and its (real) spectrum, in double.
   std::vector<double> hs(N, 0.0);
