@@ -55,6 +55,11 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -108,10 +113,10 @@ struct ColView {
 
 template <class PT>
 __device__ __forceinline__ bool col_view(const PT& P, float x, float y, float2 cs, ColView& cv) {
-  const float UU = -x * cs.x - y * cs.y;
-  const float Yr = -x * cs.y + y * cs.x;
+  const float UU = fmaf(-y, cs.y, -(x * cs.x));
+  const float Yr = fmaf(y, cs.x, -(x * cs.y));
   const float t1sq = P.SO2 - Yr * Yr;
-  const float temp1 = t1sq * rsqrtf(t1sq);
+  const float temp1 = t1sq * rsqrt_approx(t1sq);
   const float A = temp1 + UU, B = temp1 - UU;
   cv.K = P.SOSDdZL * rcp_approx(temp1 * A);
   cv.E = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
@@ -514,12 +519,12 @@ __device__ __forceinline__ void tex_column(float* __restrict__ vol, const TexRef
     if (mask == 0u) continue;
     const int p = blk.x + q;
     const float2 cs = __ldg(T.trig + p);
-    const float UU = -x * cs.x - y * cs.y;
-    const float Yr = -x * cs.y + y * cs.x;
+    const float UU = fmaf(-y, cs.y, -(x * cs.x));
+    const float Yr = fmaf(y, cs.x, -(x * cs.y));
     const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
     if (!(u1 >= 0.0f && u1 < utop)) continue;  // floor(u1) in [0, YL-2]
     const float t1sq = P.SO2 - Yr * Yr;
-    const float temp1 = t1sq * rsqrtf(t1sq);
+    const float temp1 = t1sq * rsqrt_approx(t1sq);
     const float A = temp1 + UU, B = temp1 - UU;
     const float K = P.SOSDdZL * rcp_approx(temp1 * A);
     const float E = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
@@ -567,34 +572,62 @@ __global__ void __launch_bounds__(kBx* kBy) bp_tex_kernel(float* __restrict__ vo
 // cost nothing outside their own windows. Per slice the views are visited in
 // the same order with the same operations as tex_column (a slice without the
 // view added exactly 0 there), so both give the same bits.
+//
+// V columns (x, y .. y + V - 1) per thread: what a view costs however many
+// slices hold it (loop, table and trigonometry loads, texture handle and layer,
+// the products with x) is shared by V columns, and 4 V taps are in flight. With
+// V = 1 the kernels ran into instruction issue (56 % of the slots at 55 % of
+// the filter rate on thick slices) before the texture units' rate. V = 4 with 4
+// slices, 64 registers and CTAs of 128 against the best V = 1 form, chain or
+// call: 20 rotations of 888 x 64 -> 512 x 512 x 1206 223.0 -> 205.9 ms (the
+// backprojection at 0.97 of the texture units' sample rate, was 0.89); half
+// view from host memory 38.1 -> 34.9; slabs of 3.92 mm 27.0 -> 25.8; three
+// uneven scans 68.2 -> 63.0; a 16-row head scan 2.44 -> 2.39. V = 2: 213, 35.7,
+// 26.6, 65.0, 2.44; CTAs of 64 with V = 4: 206, 35.6, 26.4, 63.6, 2.39. (Two
+// views per iteration, the earlier way to more taps in flight at thick slices,
+// was slower than V = 4 everywhere: 0.0558 against 0.0540 ms per slice on the
+// head scan, 0.2104 against 0.1956 on the slabs.)
+constexpr int kSegCols = 4;                                   // V of the several-column form
+constexpr int seg_by(int v) { return v == 1 ? kBy : kBy / 2; }  // CTA height in threads
+constexpr int kSegColsCtas = 8;                               // CTAs of 128 per SM (64 registers)
+template <int V>
 struct SegCtx {
   const float2* trig;
   const float4* btab;  // the block's first table row, two slices per float4
   const unsigned long long* texs;
-  float x, y, utop, vtop, zlch;
+  float x, y[V], utop, vtop, zlch;
   int blk0, lsh, lmask;
 };
 
-template <int NZ, int MA, int MB>
-__device__ __forceinline__ void tex_range(float (&res)[NZ], const SegCtx& c, const FastParams& P, int q0, int q1) {
+template <int NZ, int V, int MA, int MB>
+__device__ __forceinline__ void tex_range(float (&res)[V][NZ], const SegCtx<V>& c, const FastParams& P, int q0,
+                                          int q1) {
 #pragma unroll 1
   for (int q = q0; q < q1; ++q) {
     const int p = c.blk0 + q;
     const float2 cs = __ldg(c.trig + p);
-    const float UU = -c.x * cs.x - c.y * cs.y;
-    const float Yr = -c.x * cs.y + c.y * cs.x;
-    const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
-    if (!(u1 >= 0.0f && u1 < c.utop)) continue;  // floor(u1) in [0, YL-2]
-    const float t1sq = P.SO2 - Yr * Yr;
-    const float temp1 = t1sq * rsqrtf(t1sq);
-    const float A = temp1 + UU, B = temp1 - UU;
-    const float K = P.SOSDdZL * rcp_approx(temp1 * A);
-    const float E = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
+    const float xc = c.x * cs.x, xs = c.x * cs.y;
+    float K[V], E[V], xt[V];
+    bool on[V], any = false;
+#pragma unroll
+    for (int h = 0; h < V; ++h) {
+      const float UU = fmaf(-c.y[h], cs.y, -xc);
+      const float Yr = fmaf(c.y[h], cs.x, -xs);
+      const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
+      on[h] = u1 >= 0.0f && u1 < c.utop;  // floor(u1) in [0, YL-2]
+      any = any || on[h];
+      const float t1sq = P.SO2 - Yr * Yr;
+      const float temp1 = t1sq * rsqrt_approx(t1sq);
+      const float A = temp1 + UU, B = temp1 - UU;
+      K[h] = P.SOSDdZL * rcp_approx(temp1 * A);
+      E[h] = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
+      xt[h] = u1 + 0.5f;
+    }
+    if (!any) continue;
     const cudaTextureObject_t tx = __ldg(c.texs + (p >> c.lsh));
     const int layer = p & c.lmask;
-    const float xt = u1 + 0.5f;
     const float4* e = c.btab + (size_t)q * (NZ / 2);
-    float tap[NZ], qv[NZ];
+    float tap[V][NZ], qv[NZ];
 #pragma unroll
     for (int cc = MA / 2; cc <= MB / 2; ++cc) {
       const float4 t = __ldg(e + cc);  // {t2, 2^Q} of slices 2cc and 2cc+1
@@ -603,83 +636,29 @@ __device__ __forceinline__ void tex_range(float (&res)[NZ], const SegCtx& c, con
         const int m = 2 * cc + i;
         if (m < MA || m > MB) continue;
         qv[m] = i ? t.w : t.y;
-        const float vh = fmaf(i ? t.z : t.x, K, c.zlch);  // row position + 1/2
-        const bool ok = vh >= 0.5f && vh < c.vtop;
-        tap[m] = ok ? tex2DLayered<float>(tx, xt, vh, layer) : 0.0f;
-      }
-    }
 #pragma unroll
-    for (int m = MA; m <= MB; ++m) res[m] = fmaf(rcp_approx(fmaf(qv[m], E, 1.0f)), tap[m], res[m]);
-  }
-}
-
-// Two views per iteration. With thick slices few slices share a view, and one
-// view's few taps in flight per warp leave the texture units waiting on
-// latency; here both views' taps are issued before either is used. Each
-// slice still accumulates view q before view q+1 with the same operations as
-// tex_range, so the bits are the same. A view whose column misses the
-// detector is skipped as there (its per-view values are not used).
-template <int NZ, int MA, int MB>
-__device__ __forceinline__ void tex_range2(float (&res)[NZ], const SegCtx& c, const FastParams& P, int q0, int q1) {
-  int q = q0;
-#pragma unroll 1
-  for (; q + 1 < q1; q += 2) {
-    float tap[2][NZ], qv[2][NZ], E[2];
-    bool onv[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int p = c.blk0 + q + h;
-      const float2 cs = __ldg(c.trig + p);
-      const float UU = -c.x * cs.x - c.y * cs.y;
-      const float Yr = -c.x * cs.y + c.y * cs.x;
-      const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
-      onv[h] = u1 >= 0.0f && u1 < c.utop;  // floor(u1) in [0, YL-2]
-      const float t1sq = P.SO2 - Yr * Yr;
-      const float temp1 = t1sq * rsqrtf(t1sq);
-      const float A = temp1 + UU, B = temp1 - UU;
-      const float K = P.SOSDdZL * rcp_approx(temp1 * A);
-      E[h] = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
-      const cudaTextureObject_t tx = __ldg(c.texs + (p >> c.lsh));
-      const int layer = p & c.lmask;
-      const float xt = u1 + 0.5f;
-      const float4* e = c.btab + (size_t)(q + h) * (NZ / 2);
-#pragma unroll
-      for (int cc = MA / 2; cc <= MB / 2; ++cc) {
-        const float4 t = __ldg(e + cc);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int m = 2 * cc + i;
-          if (m < MA || m > MB) continue;
-          qv[h][m] = i ? t.w : t.y;
-          const float vh = fmaf(i ? t.z : t.x, K, c.zlch);
-          const bool ok = onv[h] && vh >= 0.5f && vh < c.vtop;
-          tap[h][m] = ok ? tex2DLayered<float>(tx, xt, vh, layer) : 0.0f;
+        for (int h = 0; h < V; ++h) {
+          const float vh = fmaf(i ? t.z : t.x, K[h], c.zlch);  // row position + 1/2
+          const bool ok = (V == 1 || on[h]) && vh >= 0.5f && vh < c.vtop;
+          tap[h][m] = ok ? tex2DLayered<float>(tx, xt[h], vh, layer) : 0.0f;
         }
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-      if (onv[h]) {
+    for (int h = 0; h < V; ++h)
 #pragma unroll
-        for (int m = MA; m <= MB; ++m) res[m] = fmaf(rcp_approx(fmaf(qv[h][m], E[h], 1.0f)), tap[h][m], res[m]);
+      for (int m = MA; m <= MB; ++m) {
+        const float r = fmaf(rcp_approx(fmaf(qv[m], E[h], 1.0f)), tap[h][m], res[h][m]);
+        res[h][m] = V == 1 || on[h] ? r : res[h][m];
       }
   }
-  if (q < q1) tex_range<NZ, MA, MB>(res, c, P, q, q1);  // an odd last view
 }
 
-// Widest slice range the two-view loop runs (wider ranges: one view at a
-// time, whose taps already fill the texture pipe).
-constexpr int kTwoViewMaxRange = 4;
-
-// Runs segment sg = {q0, q1, ma, mb} with the code specialised for its range
-// (V = 2: two views per iteration for ranges of at most kTwoViewMaxRange slices).
+// Runs segment sg = {q0, q1, ma, mb} with the code specialised for its range.
 template <int NZ, int V, int MA, int MB>
-__device__ __forceinline__ void tex_dispatch(float (&res)[NZ], const SegCtx& c, const FastParams& P, int4 sg) {
+__device__ __forceinline__ void tex_dispatch(float (&res)[V][NZ], const SegCtx<V>& c, const FastParams& P, int4 sg) {
   if (sg.z == MA && sg.w == MB) {
-    if constexpr (V == 2 && MB - MA + 1 <= kTwoViewMaxRange)
-      tex_range2<NZ, MA, MB>(res, c, P, sg.x, sg.y);
-    else
-      tex_range<NZ, MA, MB>(res, c, P, sg.x, sg.y);
+    tex_range<NZ, V, MA, MB>(res, c, P, sg.x, sg.y);
     return;
   }
   if constexpr (MB + 1 < NZ)
@@ -688,27 +667,30 @@ __device__ __forceinline__ void tex_dispatch(float (&res)[NZ], const SegCtx& c, 
     tex_dispatch<NZ, V, MA + 1, MA + 1>(res, c, P, sg);
 }
 
-// One column of z block b with the segmented view loop (segments in T.seg).
+// V columns (xi, yi), (xi, yi + 1) of z block b with the segmented view loop (segments in T.seg).
 template <int NZ, int V = 1>
 __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const TexRef& X, const ZTabs& T,
                                                const FastParams& P, int xi, int yi, int b) {
   static_assert(NZ % 2 == 0, "table entries are read two slices at a time");
   const int z0 = b * NZ;
-  SegCtx c;
+  SegCtx<V> c;
   c.trig = T.trig;
   c.btab = reinterpret_cast<const float4*>(T.ztab + (size_t)T.zoff[b] * NZ);
   c.texs = X.texs;
   c.x = ((float)xi - P.XNC) * P.dx;
-  c.y = ((float)yi - P.YNC) * P.dy;
+#pragma unroll
+  for (int h = 0; h < V; ++h) c.y[h] = ((float)(yi + h) - P.YNC) * P.dy;
   c.utop = (float)(P.YL - 1);
   c.vtop = (float)P.ZL - 0.5f;
   c.zlch = P.ZLC0 + 0.5f;
   c.blk0 = T.zblock[b].x;
   c.lsh = X.lsh;
   c.lmask = (1 << X.lsh) - 1;
-  float res[NZ];
+  float res[V][NZ];
 #pragma unroll
-  for (int m = 0; m < NZ; ++m) res[m] = 0.0f;
+  for (int h = 0; h < V; ++h)
+#pragma unroll
+    for (int m = 0; m < NZ; ++m) res[h][m] = 0.0f;
   const int4* sb = T.seg + (size_t)b * (hr::kSegPerNz * NZ);
 #pragma unroll 1
   for (int sgi = 0; sgi < hr::kSegPerNz * NZ; ++sgi) {
@@ -717,29 +699,33 @@ __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const Te
     tex_dispatch<NZ, V, 0, 0>(res, c, P, sg);
   }
   const float outs = P.DeltaFai * __ldg(X.scale);
-  float* out = vol + ((size_t)yi * P.XN + xi) * P.ZN + z0;
 #pragma unroll
-  for (int m = 0; m < NZ; ++m)
-    if (z0 + m < P.ZN) out[m] = res[m] * outs;
+  for (int h = 0; h < V; ++h) {
+    if (yi + h >= P.YN) break;
+    float* out = vol + ((size_t)(yi + h) * P.XN + xi) * P.ZN + z0;
+#pragma unroll
+    for (int m = 0; m < NZ; ++m)
+      if (z0 + m < P.ZN) out[m] = res[h][m] * outs;
+  }
 }
 
 template <int NZ, int V>
-__global__ void __launch_bounds__(kBx* kBy) bp_tex_seg_kernel(float* __restrict__ vol, const TexRef X, const ZTabs T,
-                                                             const FastParams P, int b_first) {
+__global__ void __launch_bounds__(kBx* seg_by(V)) bp_tex_seg_kernel(float* __restrict__ vol, const TexRef X,
+                                                                    const ZTabs T, const FastParams P, int b_first) {
   const int xi = blockIdx.x * kBx + threadIdx.x;
-  const int yi = blockIdx.y * kBy + threadIdx.y;
+  const int yi = (blockIdx.y * seg_by(V) + threadIdx.y) * V;
   if (xi >= P.XN || yi >= P.YN) return;
   tex_seg_column<NZ, V>(vol, X, T, P, xi, yi, b_first + blockIdx.z);
 }
 
-// The same column code with registers bounded for 6 CTAs of 256 threads per
-// SM (40 registers instead of 48: one CTA more per SM to hide the texture
-// latency).
+// The same column code with registers bounded: one column for 6 CTAs of 256
+// threads per SM (40 registers instead of 48), several for 8 of 128 (64 instead
+// of 72): more warps per SM to hide the texture latency.
 template <int NZ, int V>
-__global__ void __launch_bounds__(kBx* kBy, 6) bp_tex_seg6_kernel(float* __restrict__ vol, const TexRef X,
-                                                                 const ZTabs T, const FastParams P, int b_first) {
+__global__ void __launch_bounds__(kBx* seg_by(V), V == 1 ? 6 : kSegColsCtas)
+    bp_tex_seg_occ_kernel(float* __restrict__ vol, const TexRef X, const ZTabs T, const FastParams P, int b_first) {
   const int xi = blockIdx.x * kBx + threadIdx.x;
-  const int yi = blockIdx.y * kBy + threadIdx.y;
+  const int yi = (blockIdx.y * seg_by(V) + threadIdx.y) * V;
   if (xi >= P.XN || yi >= P.YN) return;
   tex_seg_column<NZ, V>(vol, X, T, P, xi, yi, b_first + blockIdx.z);
 }
@@ -1198,14 +1184,15 @@ static void launch_tex(const BpFastTables& t, const BpFast& f, const FastParams&
   bp_tex_kernel<NZ><<<grid, dim3(kBx, kBy), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
 }
 
-template <int NZ, int V>
+template <int NZ, int V, bool OCC>
 static void launch_tex_seg(const BpFastTables& t, const BpFast& f, const FastParams& P, float* vol, int b_first,
-                           int b_count, bool occ6, cudaStream_t s) {
-  dim3 grid((P.XN + kBx - 1) / kBx, (P.YN + kBy - 1) / kBy, b_count);
-  if (occ6)
-    bp_tex_seg6_kernel<NZ, V><<<grid, dim3(kBx, kBy), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
+                           int b_count, cudaStream_t s) {
+  constexpr int by = seg_by(V);
+  dim3 grid((P.XN + kBx - 1) / kBx, (P.YN + by * V - 1) / (by * V), b_count);
+  if constexpr (OCC)
+    bp_tex_seg_occ_kernel<NZ, V><<<grid, dim3(kBx, by), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
   else
-    bp_tex_seg_kernel<NZ, V><<<grid, dim3(kBx, kBy), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
+    bp_tex_seg_kernel<NZ, V><<<grid, dim3(kBx, by), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
 }
 
 // Launches variant v over z blocks [b_first, b_first + b_count) (count < 0: all).
@@ -1221,13 +1208,15 @@ static int run_variant(const BpFast& f, const BpFastGeom& g, int v, float* vol, 
     HR_REQUIRE(f.tex.kind == fv.tex && f.tex.views >= g.PN, "fast backprojection: the textures of variant %d are "
                "not prepared", v);
     if (fv.seg) {
-      const bool two = fv.seg == 2, occ6 = fv.occ == 6;
-      if (kFastNz[fv.table] == 8)
-        two ? launch_tex_seg<8, 2>(t, f, P, vol, b_first, b_count, occ6, s)
-            : launch_tex_seg<8, 1>(t, f, P, vol, b_first, b_count, occ6, s);
-      else
-        two ? launch_tex_seg<4, 2>(t, f, P, vol, b_first, b_count, occ6, s)
-            : launch_tex_seg<4, 1>(t, f, P, vol, b_first, b_count, occ6, s);
+      switch (v) {
+        case 16: launch_tex_seg<8, 1, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 17: launch_tex_seg<4, 1, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 18: launch_tex_seg<8, kSegCols, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 19: launch_tex_seg<4, kSegCols, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 20: launch_tex_seg<8, 1, true>(t, f, P, vol, b_first, b_count, s); break;
+        case 21: launch_tex_seg<4, kSegCols, true>(t, f, P, vol, b_first, b_count, s); break;
+        default: return hr::fail(HR_ERR_INVALID_ARGUMENT, "fast backprojection: unknown variant %d", v);
+      }
     } else {
       switch (kFastNz[fv.table]) {
         case 16: launch_tex<16>(t, f, P, vol, b_first, b_count, s); break;
@@ -1512,8 +1501,8 @@ int bp_fast_describe(const BpFast& f, char* buf, int len) {
   if (!buf || len <= 0) return HR_OK;
   const FastVariant& fv = kFastVariants[f.variant];
   int n = snprintf(buf, (size_t)len, "slices_per_thread=%d gathers=%s tile=%dx%d %s", kFastNz[fv.table],
-                   fv.tex == kTexHalf ? (fv.seg == 2 ? (fv.occ ? "texture-fp16-segmented-two-views-6ctas"
-                                                               : "texture-fp16-segmented-two-views")
+                   fv.tex == kTexHalf ? (fv.seg == 2 ? (fv.occ ? "texture-fp16-segmented-four-columns-8ctas"
+                                                               : "texture-fp16-segmented-four-columns")
                                         : fv.seg ? (fv.occ ? "texture-fp16-segmented-6ctas" : "texture-fp16-segmented")
                                         : "texture-fp16")
                    : fv.tex == kTexFloat ? "texture-fp32"

@@ -35,10 +35,9 @@ constexpr int kTexHalf = 1, kTexFloat = 2;
 // a z block runs in segments over which the set of slices whose window holds
 // the view is a fixed range [ma, mb], with code specialised for that range, so
 // slices without the view cost nothing (thick slices: a block's union window
-// is much longer than one slice's); seg = 2: segments whose range holds at
-// most 4 slices run two views per iteration, both views' taps in flight
-// together (thick slices: few taps per view). occ = 6: the segmented code with
-// registers bounded for 6 CTAs per SM.
+// is much longer than one slice's); seg = 2: the same with four columns per
+// thread, which share what a view costs apart from its taps. occ: registers
+// bounded for 6 CTAs per SM (seg = 1) or 8 of half the threads (seg = 2).
 struct FastVariant {
   int table, chunk, tex, seg, occ;
 };
@@ -48,7 +47,7 @@ constexpr FastVariant kFastVariants[] = {{0, 0}, {0, 4}, {0, 8}, {1, 0}, {1, 4},
                                          {1, 0, kTexFloat}, {0, 0, kTexFloat},
                                          {1, 0, kTexHalf, 1}, {2, 0, kTexHalf, 1},
                                          {1, 0, kTexHalf, 2}, {2, 0, kTexHalf, 2},
-                                         {1, 0, kTexHalf, 1, 6}, {2, 0, kTexHalf, 2, 6}};
+                                         {1, 0, kTexHalf, 1, 6}, {2, 0, kTexHalf, 2, 8}};
 constexpr int kFastVariants_n = sizeof(kFastVariants) / sizeof(kFastVariants[0]);
 constexpr int kFastDefaultVariant = 0;
 
