@@ -680,29 +680,28 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       umma_commit(mdone);
       mbar_drain(mdone, 0, err, kWaitLimit);
     }
-  } else if (lane == 0) {
-    // ---- copies: halo rows of input rows y - 1 .. y + 2, tile rows of gradient rows y, y + 1 --------
+  } else {
+    // ---- copies: halo rows of input rows y - 1 .. y + 2, tile rows of gradient rows y, y + 1, a lane to each --
+    const bool xrow = lane < 4 * XC;                                   // lanes 0 .. 4 XC - 1: (input row, group)
+    const int ln = xrow ? lane : lane - 4 * XC;                        // then (gradient row, group)
+    const int row = xrow ? ln / XC : ln / GC, c = xrow ? ln % XC : ln % GC;
+    const uint32_t dst = smem0 + (uint32_t)(xrow ? row * XC + c : kWgXPlanes + row * GC + c) * kWgPlane;
     int issued = 0;
     for (int i = 0; i < n; ++i) {
       const int s = i % kWgStages;
-      if (i >= kWgStages && !mbar_wait(&empty[s], (uint32_t)(i / kWgStages - 1) & 1, abort_flag, err, kWaitLimit))
-        break;
+      const bool free = lane != 0 || i < kWgStages ||
+                        mbar_wait(&empty[s], (uint32_t)(i / kWgStages - 1) & 1, abort_flag, err, kWaitLimit);
+      if (!__all_sync(0xffffffffu, free)) break;
       const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / nseg;
       const int x0 = (int)(t - by * nseg) * kTileM, b = (int)(by / npair), y = 2 * (int)(by - (uint32_t)b * npair);
-      const uint32_t st = smem0 + s * kWgStage;
-      mbar_expect_tx(&full[s], 4 * XC * kBox + 2 * GC * kTileM * 16);
-      for (int row = 0; row < 4; ++row) {
-        const int yy = y + row - 1;
-        const bool in = yy >= 0 && yy < H;
-        const uint4* src = in ? X + plane_row(b, H, yy, XC, 0, Wp) + x0 : zero;
-        for (int c = 0; c < XC; ++c)
-          bulk_load(st + (row * XC + c) * kWgPlane, src + (in ? (size_t)c * Wp : 0), kBox, &full[s]);
-      }
-      for (int row = 0; row < 2; ++row) {
-        const bool in = y + row < H;
-        const uint4* src = in ? Gr + plane_row(b, H, y + row, GC, 0, Wp) + x0 + 1 : zero;
-        for (int c = 0; c < GC; ++c)
-          bulk_load(st + (kWgXPlanes + row * GC + c) * kWgPlane, src + (in ? (size_t)c * Wp : 0), kTileM * 16, &full[s]);
+      if (lane == 0) mbar_expect_tx(&full[s], 4 * XC * kBox + 2 * GC * kTileM * 16);
+      __syncwarp();
+      if (lane < 4 * XC + 2 * GC) {
+        const int yy = xrow ? y + row - 1 : y + row;
+        const uint4* src = zero;
+        if (yy >= 0 && yy < H)
+          src = xrow ? X + plane_row(b, H, yy, XC, c, Wp) + x0 : Gr + plane_row(b, H, yy, GC, c, Wp) + x0 + 1;
+        bulk_load(dst + (uint32_t)s * kWgStage, src, xrow ? kBox : kTileM * 16, &full[s]);
       }
       issued = i + 1;
     }
