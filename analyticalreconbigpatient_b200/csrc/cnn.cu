@@ -161,6 +161,16 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
+// The convolution and weight-gradient kernels are launched as programmatic dependents: when the last CTA of the
+// previous kernel has ended, this one's start, set up their barriers and take TMEM while that kernel's writes are
+// still being flushed. No thread reads or writes global memory before this returns: the previous kernel is then
+// complete and its writes visible. 64 slices of 512 x 512 in two chunks 3.06 -> 2.98 ms, slice by slice 11.9 ->
+// 9.7, a training step of eight 2.00 -> 1.96. (With a trigger before a kernel's end, so that CTAs move in as
+// others leave, the column strips of a row no longer run together: 3.10 and 2.03 ms.)
+__device__ __forceinline__ void after_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Untiled bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned), reported to `bar`.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -337,10 +347,6 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
   float* bias_s = reinterpret_cast<float*>(tmem_slot + 4);  // 16-byte aligned, COUT floats
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < kWBytes / 16; i += kThreads)
-    reinterpret_cast<uint4*>(wsm)[i] = __ldg(reinterpret_cast<const uint4*>(a.wimg) + i);
-  if (tid < COUT) bias_s[tid] = a.bias ? __ldg(a.bias + tid) : 0.0f;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (tid == 0) {
     for (int s = 0; s < kRing; ++s) {
       mbar_init(&full[s], 1);
@@ -359,6 +365,11 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
                  "r"(tmem_cols(COUT)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  after_previous_kernel();
+  for (int i = tid; i < kWBytes / 16; i += kThreads)
+    reinterpret_cast<uint4*>(wsm)[i] = __ldg(reinterpret_cast<const uint4*>(a.wimg) + i);
+  if (tid < COUT) bias_s[tid] = a.bias ? __ldg(a.bias + tid) : 0.0f;
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
@@ -558,6 +569,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
                  "r"(kWgTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  after_previous_kernel();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -853,6 +865,23 @@ __global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* _
   }
 }
 
+// Launches a kernel that calls after_previous_kernel.
+template <class... P, class... A>
+int launch_dependent(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  HR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+  return HR_OK;
+}
+
 // Dynamic shared memory of a conv CTA: input-row ring + weights + barriers + alignment slack.
 template <int CIN, int COUT>
 constexpr size_t conv_smem() {
@@ -885,9 +914,7 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
   const long long groups = std::min(((long long)a.B * a.H + 3) / 4, std::max(1LL, ctas / nseg));
   const long long grid = groups * nseg;
   if (grid <= 0) return HR_OK;
-  conv_tc_kernel<CIN, COUT, EPI><<<(unsigned)grid, kThreads, smem, s>>>(a);
-  HR_CUDA_TRY(cudaGetLastError());
-  return HR_OK;
+  return launch_dependent(conv_tc_kernel<CIN, COUT, EPI>, (unsigned)grid, kThreads, smem, s, a);
 }
 
 template <int CIN, int COUT>
@@ -899,9 +926,8 @@ int launch_wgrad(const uint4* X, const uint4* Gr, const uint4* zero, int B, int 
   HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
   HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kWgSmem));
-  wgrad_tc_kernel<CIN, COUT><<<(unsigned)grid, kWgThreads, kWgSmem, s>>>(X, Gr, zero, B, H, W, dW, db, err);
-  HR_CUDA_TRY(cudaGetLastError());
-  return HR_OK;
+  return launch_dependent(wgrad_tc_kernel<CIN, COUT>, (unsigned)grid, kWgThreads, kWgSmem, s, X, Gr, zero, B, H, W,
+                          dW, db, err);
 }
 
 }  // namespace

@@ -46,3 +46,24 @@ def test_volume_equals_its_slices(cuda, H, W, ZN, chunk):
     net.check()
     assert torch.equal(out.permute(2, 0, 1), ref)  # the same sums and one fused multiply-add per pixel
     net.close()
+
+
+def test_volume_under_graph_capture(cuda):
+    """The kernels are launched as programmatic dependents of one another: captured and replayed, they wait for
+    one another as in a stream (two chunks, so that every buffer is written twice)."""
+    g = torch.Generator(device=cuda).manual_seed(9)
+    vol = (MU_WATER * (1.0 + 0.1 * torch.randn((40, 150, 12), device=cuda, generator=g))).contiguous()
+    net = L.Corrector(C.init_params(3, zero_last=False))
+    ref = net.apply_volume(vol, chunk=7).clone()
+    out = torch.zeros_like(vol)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        net.apply_volume(vol, out, chunk=7)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    net.check()
+    del graph
+    net.close()
