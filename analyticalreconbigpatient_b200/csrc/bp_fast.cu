@@ -419,8 +419,19 @@ __global__ void __launch_bounds__(kBx* kBy, MB) bp_fast_batch_kernel(const __gri
 // like unsigned integers), for the FP16 scale.
 __global__ void tex_absmax_kernel(float* __restrict__ scale, const uint32_t* __restrict__ fpb, long long n) {
   unsigned m = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    m = max(m, (__ldg(fpb + i) << 16) & 0x7fffffffu);
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  long long done = 0;
+  if ((reinterpret_cast<uintptr_t>(fpb) & 15) == 0) {
+    const uint4* f4 = reinterpret_cast<const uint4*>(fpb);
+    done = n & ~3LL;
+#pragma unroll 4
+    for (long long i = t; i < done / 4; i += nt) {
+      const uint4 w = __ldg(f4 + i);
+      m = max(max(m, (w.x << 16) & 0x7fffffffu), (w.y << 16) & 0x7fffffffu);
+      m = max(max(m, (w.z << 16) & 0x7fffffffu), (w.w << 16) & 0x7fffffffu);
+    }
+  }
+  for (long long i = done + t; i < n; i += nt) m = max(m, (__ldg(fpb + i) << 16) & 0x7fffffffu);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0 && m) atomicMax(reinterpret_cast<unsigned*>(scale + 1), m);
 }
@@ -438,6 +449,15 @@ __global__ void tex_absmax_kernel(float* __restrict__ scale, const uint32_t* __r
 // two that keeps the values in FP16's normal range gives the same samples up
 // to that power.
 constexpr int kStreamHeadroom = 4;  // binades between the first range's largest |value| and MODE 0's range
+//
+// Rows of a multiple of eight channels that start on 16-byte boundaries go by
+// CTAs of one row and threads of eight channels, four rows to an iteration: 16
+// bytes in and out per access, many in flight, and no division per texel group
+// (4.4 GB of pairs, 888 x 64 x 19,526 views: 2.67 -> 1.23 ms; the largest |value|
+// with 16-byte loads 0.91 -> 0.73). The four rows are consecutive ones: an
+// array's 32-byte sectors hold two rows' texels, and stores to rows that other
+// CTAs hold left them half written (2.81 ms).
+constexpr int kFillRows = 4;
 template <bool HALF, int MODE>
 __global__ void tex_fill_kernel(float* __restrict__ scale, const unsigned long long* __restrict__ surfs,
                                 const uint32_t* __restrict__ fpb, long long r0, long long r1, int ZL, int YL,
@@ -461,21 +481,36 @@ __global__ void tex_fill_kernel(float* __restrict__ scale, const unsigned long l
     if (blockIdx.x == 0 && threadIdx.x == 0) scale[0] = 1.0f;
   }
   const int lmask = (1 << lsh) - 1;
-  if (HALF && (YL & 3) == 0 && (reinterpret_cast<uintptr_t>(fpb) & 15) == 0) {
-    // four channels per thread: one 16-byte load of their pairs (rows start 16-byte aligned), one 8-byte
-    // (four-texel) surface store
-    const int G = YL >> 2;
-    const long long n = (r1 - r0) * G;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
-      const long long r = r0 + i / G;
-      const int g = (int)(i - (r - r0) * G);
-      const int p = (int)(r / ZL), v = (int)(r - (long long)p * ZL);
-      const uint4 w = __ldg(reinterpret_cast<const uint4*>(fpb + r * YL) + g);
-      const __half2 h01 = __floats2half2_rn(__uint_as_float(w.x << 16) * sc, __uint_as_float(w.y << 16) * sc);
-      const __half2 h23 = __floats2half2_rn(__uint_as_float(w.z << 16) * sc, __uint_as_float(w.w << 16) * sc);
-      const uint2 out = make_uint2(*reinterpret_cast<const uint32_t*>(&h01), *reinterpret_cast<const uint32_t*>(&h23));
-      surf2DLayeredwrite(out, surfs[p >> lsh], g * 8, v, p & lmask, cudaBoundaryModeZero);
+  if (HALF && (YL & 7) == 0 && r1 < (1LL << 31) && (reinterpret_cast<uintptr_t>(fpb) & 15) == 0) {
+    for (long long rb = r0 + (long long)kFillRows * blockIdx.x; rb < r1; rb += (long long)kFillRows * gridDim.x) {
+      for (int g = threadIdx.x; g < YL >> 3; g += blockDim.x) {
+        uint4 w[kFillRows][2];
+#pragma unroll
+        for (int k = 0; k < kFillRows; ++k) {
+          const long long r = rb + k;
+          if (r >= r1) continue;
+          const uint4* src = reinterpret_cast<const uint4*>(fpb + r * YL) + 2 * g;
+          w[k][0] = __ldg(src);
+          w[k][1] = __ldg(src + 1);
+        }
+#pragma unroll
+        for (int k = 0; k < kFillRows; ++k) {
+          const long long r = rb + k;
+          if (r >= r1) continue;
+          const int p = (int)((unsigned)r / (unsigned)ZL), v = (int)((unsigned)r - (unsigned)p * (unsigned)ZL);
+          uint32_t o[4];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint4 q = w[k][i];
+            const __half2 h01 = __floats2half2_rn(__uint_as_float(q.x << 16) * sc, __uint_as_float(q.y << 16) * sc);
+            const __half2 h23 = __floats2half2_rn(__uint_as_float(q.z << 16) * sc, __uint_as_float(q.w << 16) * sc);
+            o[2 * i] = *reinterpret_cast<const uint32_t*>(&h01);
+            o[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h23);
+          }
+          surf2DLayeredwrite(make_uint4(o[0], o[1], o[2], o[3]), surfs[p >> lsh], g * 16, v, p & lmask,
+                             cudaBoundaryModeZero);
+        }
+      }
     }
     return;
   }
@@ -578,18 +613,28 @@ __global__ void __launch_bounds__(kBx* kBy) bp_tex_kernel(float* __restrict__ vo
 // the products with x) is shared by V columns, and 4 V taps are in flight. With
 // V = 1 the kernels ran into instruction issue (56 % of the slots at 55 % of
 // the filter rate on thick slices) before the texture units' rate. V = 4 with 4
-// slices, 64 registers and CTAs of 128 against the best V = 1 form, chain or
-// call: 20 rotations of 888 x 64 -> 512 x 512 x 1206 223.0 -> 205.9 ms (the
+// slices, 64 registers and CTAs of 128 against the best one-column form, chain
+// or call: 20 rotations of 888 x 64 -> 512 x 512 x 1206 223.0 -> 205.9 ms (the
 // backprojection at 0.97 of the texture units' sample rate, was 0.89); half
 // view from host memory 38.1 -> 34.9; slabs of 3.92 mm 27.0 -> 25.8; three
-// uneven scans 68.2 -> 63.0; a 16-row head scan 2.44 -> 2.39. V = 2: 213, 35.7,
-// 26.6, 65.0, 2.44; CTAs of 64 with V = 4: 206, 35.6, 26.4, 63.6, 2.39. (Two
-// views per iteration, the earlier way to more taps in flight at thick slices,
-// was slower than V = 4 everywhere: 0.0558 against 0.0540 ms per slice on the
-// head scan, 0.2104 against 0.1956 on the slabs.)
-constexpr int kSegCols = 4;                                   // V of the several-column form
-constexpr int seg_by(int v) { return v == 1 ? kBy : kBy / 2; }  // CTA height in threads
-constexpr int kSegColsCtas = 8;                               // CTAs of 128 per SM (64 registers)
+// uneven scans 68.2 -> 63.0. V = 2: 213, 35.7, 26.6, 65.0; CTAs of 64 with V =
+// 4: 206, 35.6, 26.4, 63.6. Launches too small for it (several_columns) run one
+// column and, in narrow segments, two views at a time.
+constexpr int kSegCols = 4;      // V of the several-column form
+constexpr int kSegColsCtas = 8;  // CTAs of 128 per SM (64 registers)
+// Threads of a CTA, its tile (x, y) and a thread's column (the first of its V). Warps are 8 x 4 threads; the
+// several-column form's four lie two by two, so that its tile is as high as the other's and a grid's edge
+// leaves as little of it empty.
+constexpr int seg_threads(int v) { return v == 1 ? kBx * kBy : kBx * kBy / 2; }
+constexpr int seg_tile_x(int v) { return v == 1 ? kBx : 2 * kBx; }
+constexpr int seg_tile_y(int v) { return v == 1 ? kBy : 8 * v; }
+template <int V>
+__device__ __forceinline__ int2 seg_thread_column() {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wx = V == 1 ? 0 : warp & 1, wy = V == 1 ? warp : warp >> 1;
+  return make_int2(blockIdx.x * seg_tile_x(V) + wx * 8 + (lane & 7),
+                   blockIdx.y * seg_tile_y(V) + (wy * 4 + (lane >> 3)) * V);
+}
 template <int V>
 struct SegCtx {
   const float2* trig;
@@ -654,21 +699,83 @@ __device__ __forceinline__ void tex_range(float (&res)[V][NZ], const SegCtx<V>& 
   }
 }
 
-// Runs segment sg = {q0, q1, ma, mb} with the code specialised for its range.
-template <int NZ, int V, int MA, int MB>
+// Two views per iteration, for one column: with thick slices few slices share a
+// view, and where a launch is too small for several columns per thread the
+// second view's taps fill the wait for the first's. Each slice still
+// accumulates view q before view q + 1 with the same operations.
+template <int NZ, int MA, int MB>
+__device__ __forceinline__ void tex_range2(float (&res)[1][NZ], const SegCtx<1>& c, const FastParams& P, int q0,
+                                           int q1) {
+  int q = q0;
+#pragma unroll 1
+  for (; q + 1 < q1; q += 2) {
+    float tap[2][NZ], qv[2][NZ], E[2];
+    bool onv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = c.blk0 + q + h;
+      const float2 cs = __ldg(c.trig + p);
+      const float UU = fmaf(-c.y[0], cs.y, -(c.x * cs.x));
+      const float Yr = fmaf(c.y[0], cs.x, -(c.x * cs.y));
+      const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
+      onv[h] = u1 >= 0.0f && u1 < c.utop;  // floor(u1) in [0, YL-2]
+      const float t1sq = P.SO2 - Yr * Yr;
+      const float temp1 = t1sq * rsqrt_approx(t1sq);
+      const float A = temp1 + UU, B = temp1 - UU;
+      const float K = P.SOSDdZL * rcp_approx(temp1 * A);
+      E[h] = ex2_approx(P.k1 * lg2_approx(B * rcp_approx(A)));
+      const cudaTextureObject_t tx = __ldg(c.texs + (p >> c.lsh));
+      const int layer = p & c.lmask;
+      const float xt = u1 + 0.5f;
+      const float4* e = c.btab + (size_t)(q + h) * (NZ / 2);
+#pragma unroll
+      for (int cc = MA / 2; cc <= MB / 2; ++cc) {
+        const float4 t = __ldg(e + cc);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int m = 2 * cc + i;
+          if (m < MA || m > MB) continue;
+          qv[h][m] = i ? t.w : t.y;
+          const float vh = fmaf(i ? t.z : t.x, K, c.zlch);
+          const bool ok = onv[h] && vh >= 0.5f && vh < c.vtop;
+          tap[h][m] = ok ? tex2DLayered<float>(tx, xt, vh, layer) : 0.0f;
+        }
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (onv[h]) {
+#pragma unroll
+        for (int m = MA; m <= MB; ++m)
+          res[0][m] = fmaf(rcp_approx(fmaf(qv[h][m], E[h], 1.0f)), tap[h][m], res[0][m]);
+      }
+  }
+  if (q < q1) tex_range<NZ, 1, MA, MB>(res, c, P, q, q1);  // an odd last view
+}
+
+// Widest slice range the two-view loop runs (wider ranges: one view at a
+// time, whose taps already fill the texture pipe).
+constexpr int kTwoViewMaxRange = 4;
+
+// Runs segment sg = {q0, q1, ma, mb} with the code specialised for its range
+// (VIEWS = 2: two views per iteration for ranges of at most kTwoViewMaxRange slices).
+template <int NZ, int V, int VIEWS, int MA, int MB>
 __device__ __forceinline__ void tex_dispatch(float (&res)[V][NZ], const SegCtx<V>& c, const FastParams& P, int4 sg) {
   if (sg.z == MA && sg.w == MB) {
-    tex_range<NZ, V, MA, MB>(res, c, P, sg.x, sg.y);
+    if constexpr (V == 1 && VIEWS == 2 && MB - MA + 1 <= kTwoViewMaxRange)
+      tex_range2<NZ, MA, MB>(res, c, P, sg.x, sg.y);
+    else
+      tex_range<NZ, V, MA, MB>(res, c, P, sg.x, sg.y);
     return;
   }
   if constexpr (MB + 1 < NZ)
-    tex_dispatch<NZ, V, MA, MB + 1>(res, c, P, sg);
+    tex_dispatch<NZ, V, VIEWS, MA, MB + 1>(res, c, P, sg);
   else if constexpr (MA + 1 < NZ)
-    tex_dispatch<NZ, V, MA + 1, MA + 1>(res, c, P, sg);
+    tex_dispatch<NZ, V, VIEWS, MA + 1, MA + 1>(res, c, P, sg);
 }
 
 // V columns (xi, yi), (xi, yi + 1) of z block b with the segmented view loop (segments in T.seg).
-template <int NZ, int V = 1>
+template <int NZ, int V = 1, int VIEWS = 1>
 __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const TexRef& X, const ZTabs& T,
                                                const FastParams& P, int xi, int yi, int b) {
   static_assert(NZ % 2 == 0, "table entries are read two slices at a time");
@@ -696,7 +803,7 @@ __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const Te
   for (int sgi = 0; sgi < hr::kSegPerNz * NZ; ++sgi) {
     const int4 sg = __ldg(sb + sgi);
     if (sg.x >= sg.y) continue;  // unused entry (uniform over the CTA)
-    tex_dispatch<NZ, V, 0, 0>(res, c, P, sg);
+    tex_dispatch<NZ, V, VIEWS, 0, 0>(res, c, P, sg);
   }
   const float outs = P.DeltaFai * __ldg(X.scale);
 #pragma unroll
@@ -709,25 +816,23 @@ __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const Te
   }
 }
 
-template <int NZ, int V>
-__global__ void __launch_bounds__(kBx* seg_by(V)) bp_tex_seg_kernel(float* __restrict__ vol, const TexRef X,
+template <int NZ, int V, int VIEWS>
+__global__ void __launch_bounds__(seg_threads(V)) bp_tex_seg_kernel(float* __restrict__ vol, const TexRef X,
                                                                     const ZTabs T, const FastParams P, int b_first) {
-  const int xi = blockIdx.x * kBx + threadIdx.x;
-  const int yi = (blockIdx.y * seg_by(V) + threadIdx.y) * V;
-  if (xi >= P.XN || yi >= P.YN) return;
-  tex_seg_column<NZ, V>(vol, X, T, P, xi, yi, b_first + blockIdx.z);
+  const int2 c = seg_thread_column<V>();
+  if (c.x >= P.XN || c.y >= P.YN) return;
+  tex_seg_column<NZ, V, VIEWS>(vol, X, T, P, c.x, c.y, b_first + blockIdx.z);
 }
 
 // The same column code with registers bounded: one column for 6 CTAs of 256
 // threads per SM (40 registers instead of 48), several for 8 of 128 (64 instead
 // of 72): more warps per SM to hide the texture latency.
-template <int NZ, int V>
-__global__ void __launch_bounds__(kBx* seg_by(V), V == 1 ? 6 : kSegColsCtas)
+template <int NZ, int V, int VIEWS>
+__global__ void __launch_bounds__(seg_threads(V), V == 1 ? 6 : kSegColsCtas)
     bp_tex_seg_occ_kernel(float* __restrict__ vol, const TexRef X, const ZTabs T, const FastParams P, int b_first) {
-  const int xi = blockIdx.x * kBx + threadIdx.x;
-  const int yi = (blockIdx.y * seg_by(V) + threadIdx.y) * V;
-  if (xi >= P.XN || yi >= P.YN) return;
-  tex_seg_column<NZ, V>(vol, X, T, P, xi, yi, b_first + blockIdx.z);
+  const int2 c = seg_thread_column<V>();
+  if (c.x >= P.XN || c.y >= P.YN) return;
+  tex_seg_column<NZ, V, VIEWS>(vol, X, T, P, c.x, c.y, b_first + blockIdx.z);
 }
 
 // The persistent multi-scan launch with texture taps: the work items and
@@ -1111,15 +1216,16 @@ int bp_fast_tex_fill_range(const BpFast& f, const BpFastGeom& g, const uint32_t*
              "[%d, %d) (mode %d) outside [0, %d)", p0, p1, mode, g.PN);
   const long long r0 = (long long)p0 * g.ZL, r1 = (long long)p1 * g.ZL;
   const int grid = (int)std::max(1LL, std::min<long long>(r1 - r0, 16LL * sm_count()));
+  const int threads = 128;  // a CTA takes whole rows: 888 channels in groups of eight are 111 threads' work
   if (t.kind == kTexHalf) {
     if (mode != 2) HR_CUDA_TRY(cudaMemsetAsync(t.d_scale + 1, 0, sizeof(float), s));
-    if (r1 > r0) tex_absmax_kernel<<<4 * sm_count(), 256, 0, s>>>(t.d_scale, fpb + r0 * g.YL, (r1 - r0) * g.YL);
+    if (r1 > r0) tex_absmax_kernel<<<8 * sm_count(), 256, 0, s>>>(t.d_scale, fpb + r0 * g.YL, (r1 - r0) * g.YL);
     if (mode == 0)
-      tex_fill_kernel<true, 0><<<grid, 256, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
+      tex_fill_kernel<true, 0><<<grid, threads, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
     else if (mode == 1)
-      tex_fill_kernel<true, 1><<<grid, 256, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
+      tex_fill_kernel<true, 1><<<grid, threads, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
     else
-      tex_fill_kernel<true, 2><<<grid, 256, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
+      tex_fill_kernel<true, 2><<<grid, threads, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
   } else {
     if (mode == 1) HR_CUDA_TRY(cudaMemsetAsync(t.d_scale + 3, 0, sizeof(float), s));
     tex_fill_kernel<false, 0><<<grid, 256, 0, s>>>(t.d_scale, t.d_obj + t.n, fpb, r0, r1, g.ZL, g.YL, t.lsh);
@@ -1184,15 +1290,29 @@ static void launch_tex(const BpFastTables& t, const BpFast& f, const FastParams&
   bp_tex_kernel<NZ><<<grid, dim3(kBx, kBy), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
 }
 
-template <int NZ, int V, bool OCC>
+template <int NZ, int V, int VIEWS, bool OCC>
 static void launch_tex_seg(const BpFastTables& t, const BpFast& f, const FastParams& P, float* vol, int b_first,
                            int b_count, cudaStream_t s) {
-  constexpr int by = seg_by(V);
-  dim3 grid((P.XN + kBx - 1) / kBx, (P.YN + by * V - 1) / (by * V), b_count);
+  dim3 grid((P.XN + seg_tile_x(V) - 1) / seg_tile_x(V), (P.YN + seg_tile_y(V) - 1) / seg_tile_y(V), b_count);
   if constexpr (OCC)
-    bp_tex_seg_occ_kernel<NZ, V><<<grid, dim3(kBx, by), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
+    bp_tex_seg_occ_kernel<NZ, V, VIEWS><<<grid, seg_threads(V), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
   else
-    bp_tex_seg_kernel<NZ, V><<<grid, dim3(kBx, by), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
+    bp_tex_seg_kernel<NZ, V, VIEWS><<<grid, seg_threads(V), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
+}
+
+// Whether a launch over z blocks [b_first, b_first + b_count) has the CTAs for kSegCols columns per thread: two
+// rounds of them, blocks without views not counted. Fewer leave SMs idle at the end, and beside another kernel (a
+// slab's or chunk's filter) one round of long CTAs keeps that kernel out until it ends. Measured, several columns
+// against two views: 512 x 512 x 16 (1.7 rounds) 4.80 / 5.00 ms, 301 x 301 x 40 (1.6) 4.64 / 4.71, 256 x 256 x 24
+// (0.6) 1.82 / 1.82, 200 x 200 x 64 (1.2) 3.86 / 3.71, 130 x 130 x 128 (1.2) 2.65 / 2.48; slabs of 256 x 256 x 32
+// (0.9, filter beside it) 30.8 / 28.7.
+static bool several_columns(const BpFastTables& t, const FastParams& P, int b_first, int b_count) {
+  long long blocks = 0;
+  for (int b = b_first; b < b_first + b_count; ++b)
+    if (t.h_zb.size() < 2 * (size_t)t.nblocks || t.h_zb[2 * b + 1] > 0) ++blocks;
+  const long long tiles = (long long)((P.XN + seg_tile_x(kSegCols) - 1) / seg_tile_x(kSegCols)) *
+                          ((P.YN + seg_tile_y(kSegCols) - 1) / seg_tile_y(kSegCols));
+  return tiles * blocks >= 2LL * kSegColsCtas * sm_count();
 }
 
 // Launches variant v over z blocks [b_first, b_first + b_count) (count < 0: all).
@@ -1208,13 +1328,23 @@ static int run_variant(const BpFast& f, const BpFastGeom& g, int v, float* vol, 
     HR_REQUIRE(f.tex.kind == fv.tex && f.tex.views >= g.PN, "fast backprojection: the textures of variant %d are "
                "not prepared", v);
     if (fv.seg) {
+      const bool cols = fv.seg == 2 && several_columns(t, P, b_first, b_count);
       switch (v) {
-        case 16: launch_tex_seg<8, 1, false>(t, f, P, vol, b_first, b_count, s); break;
-        case 17: launch_tex_seg<4, 1, false>(t, f, P, vol, b_first, b_count, s); break;
-        case 18: launch_tex_seg<8, kSegCols, false>(t, f, P, vol, b_first, b_count, s); break;
-        case 19: launch_tex_seg<4, kSegCols, false>(t, f, P, vol, b_first, b_count, s); break;
-        case 20: launch_tex_seg<8, 1, true>(t, f, P, vol, b_first, b_count, s); break;
-        case 21: launch_tex_seg<4, kSegCols, true>(t, f, P, vol, b_first, b_count, s); break;
+        case 16: launch_tex_seg<8, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 17: launch_tex_seg<4, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
+        case 18:
+          cols ? launch_tex_seg<8, kSegCols, 1, false>(t, f, P, vol, b_first, b_count, s)
+               : launch_tex_seg<8, 1, 2, false>(t, f, P, vol, b_first, b_count, s);
+          break;
+        case 19:
+          cols ? launch_tex_seg<4, kSegCols, 1, false>(t, f, P, vol, b_first, b_count, s)
+               : launch_tex_seg<4, 1, 2, false>(t, f, P, vol, b_first, b_count, s);
+          break;
+        case 20: launch_tex_seg<8, 1, 1, true>(t, f, P, vol, b_first, b_count, s); break;
+        case 21:
+          cols ? launch_tex_seg<4, kSegCols, 1, true>(t, f, P, vol, b_first, b_count, s)
+               : launch_tex_seg<4, 1, 2, true>(t, f, P, vol, b_first, b_count, s);
+          break;
         default: return hr::fail(HR_ERR_INVALID_ARGUMENT, "fast backprojection: unknown variant %d", v);
       }
     } else {

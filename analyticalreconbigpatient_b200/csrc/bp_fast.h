@@ -36,8 +36,10 @@ constexpr int kTexHalf = 1, kTexFloat = 2;
 // the view is a fixed range [ma, mb], with code specialised for that range, so
 // slices without the view cost nothing (thick slices: a block's union window
 // is much longer than one slice's); seg = 2: the same with four columns per
-// thread, which share what a view costs apart from its taps. occ: registers
-// bounded for 6 CTAs per SM (seg = 1) or 8 of half the threads (seg = 2).
+// thread, which share what a view costs apart from its taps, or, in launches
+// too small for that, with two views per iteration in segments of at most four
+// slices. occ: registers bounded for 6 CTAs per SM (8 of half the threads with
+// four columns).
 struct FastVariant {
   int table, chunk, tex, seg, occ;
 };
