@@ -450,14 +450,52 @@ __global__ void tex_absmax_kernel(float* __restrict__ scale, const uint32_t* __r
 // to that power.
 constexpr int kStreamHeadroom = 4;  // binades between the first range's largest |value| and MODE 0's range
 //
-// Rows of a multiple of eight channels that start on 16-byte boundaries go by
-// CTAs of one row and threads of eight channels, four rows to an iteration: 16
+// Rows of a multiple of eight (or four) channels that start on 16-byte boundaries
+// go by CTAs of four rows and threads of eight (four) channels: 16
 // bytes in and out per access, many in flight, and no division per texel group
 // (4.4 GB of pairs, 888 x 64 x 19,526 views: 2.67 -> 1.23 ms; the largest |value|
 // with 16-byte loads 0.91 -> 0.73). The four rows are consecutive ones: an
 // array's 32-byte sectors hold two rows' texels, and stores to rows that other
 // CTAs hold left them half written (2.81 ms).
 constexpr int kFillRows = 4;
+template <int C>  // channels per thread: 8 or 4
+__device__ __forceinline__ void fill_rows(const unsigned long long* __restrict__ surfs, const uint32_t* __restrict__ fpb,
+                                          long long r0, long long r1, int ZL, int YL, int lsh, float sc) {
+  const int lmask = (1 << lsh) - 1;
+  for (long long rb = r0 + (long long)kFillRows * blockIdx.x; rb < r1; rb += (long long)kFillRows * gridDim.x) {
+    for (int g = threadIdx.x; g < YL / C; g += blockDim.x) {
+      uint4 w[kFillRows][C / 4];
+#pragma unroll
+      for (int k = 0; k < kFillRows; ++k) {
+        if (rb + k >= r1) continue;
+#pragma unroll
+        for (int i = 0; i < C / 4; ++i)
+          w[k][i] = __ldg(reinterpret_cast<const uint4*>(fpb + (rb + k) * YL) + C / 4 * g + i);
+      }
+#pragma unroll
+      for (int k = 0; k < kFillRows; ++k) {
+        if (rb + k >= r1) continue;
+        const unsigned r = (unsigned)(rb + k), p = r / (unsigned)ZL, v = r - p * (unsigned)ZL;
+        uint32_t o[C / 2];
+#pragma unroll
+        for (int i = 0; i < C / 4; ++i) {
+          const uint4 q = w[k][i];
+          const __half2 h01 = __floats2half2_rn(__uint_as_float(q.x << 16) * sc, __uint_as_float(q.y << 16) * sc);
+          const __half2 h23 = __floats2half2_rn(__uint_as_float(q.z << 16) * sc, __uint_as_float(q.w << 16) * sc);
+          o[2 * i] = *reinterpret_cast<const uint32_t*>(&h01);
+          o[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h23);
+        }
+        if constexpr (C == 8)
+          surf2DLayeredwrite(make_uint4(o[0], o[1], o[2], o[3]), surfs[p >> lsh], g * 16, (int)v, (int)p & lmask,
+                             cudaBoundaryModeZero);
+        else
+          surf2DLayeredwrite(make_uint2(o[0], o[1]), surfs[p >> lsh], g * 8, (int)v, (int)p & lmask,
+                             cudaBoundaryModeZero);
+      }
+    }
+  }
+}
+
 template <bool HALF, int MODE>
 __global__ void tex_fill_kernel(float* __restrict__ scale, const unsigned long long* __restrict__ surfs,
                                 const uint32_t* __restrict__ fpb, long long r0, long long r1, int ZL, int YL,
@@ -481,37 +519,11 @@ __global__ void tex_fill_kernel(float* __restrict__ scale, const unsigned long l
     if (blockIdx.x == 0 && threadIdx.x == 0) scale[0] = 1.0f;
   }
   const int lmask = (1 << lsh) - 1;
-  if (HALF && (YL & 7) == 0 && r1 < (1LL << 31) && (reinterpret_cast<uintptr_t>(fpb) & 15) == 0) {
-    for (long long rb = r0 + (long long)kFillRows * blockIdx.x; rb < r1; rb += (long long)kFillRows * gridDim.x) {
-      for (int g = threadIdx.x; g < YL >> 3; g += blockDim.x) {
-        uint4 w[kFillRows][2];
-#pragma unroll
-        for (int k = 0; k < kFillRows; ++k) {
-          const long long r = rb + k;
-          if (r >= r1) continue;
-          const uint4* src = reinterpret_cast<const uint4*>(fpb + r * YL) + 2 * g;
-          w[k][0] = __ldg(src);
-          w[k][1] = __ldg(src + 1);
-        }
-#pragma unroll
-        for (int k = 0; k < kFillRows; ++k) {
-          const long long r = rb + k;
-          if (r >= r1) continue;
-          const int p = (int)((unsigned)r / (unsigned)ZL), v = (int)((unsigned)r - (unsigned)p * (unsigned)ZL);
-          uint32_t o[4];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const uint4 q = w[k][i];
-            const __half2 h01 = __floats2half2_rn(__uint_as_float(q.x << 16) * sc, __uint_as_float(q.y << 16) * sc);
-            const __half2 h23 = __floats2half2_rn(__uint_as_float(q.z << 16) * sc, __uint_as_float(q.w << 16) * sc);
-            o[2 * i] = *reinterpret_cast<const uint32_t*>(&h01);
-            o[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&h23);
-          }
-          surf2DLayeredwrite(make_uint4(o[0], o[1], o[2], o[3]), surfs[p >> lsh], g * 16, v, p & lmask,
-                             cudaBoundaryModeZero);
-        }
-      }
-    }
+  if (HALF && (YL & 3) == 0 && r1 < (1LL << 31) && (reinterpret_cast<uintptr_t>(fpb) & 15) == 0) {
+    if ((YL & 7) == 0)
+      fill_rows<8>(surfs, fpb, r0, r1, ZL, YL, lsh, sc);
+    else
+      fill_rows<4>(surfs, fpb, r0, r1, ZL, YL, lsh, sc);
     return;
   }
   for (long long r = r0 + blockIdx.x; r < r1; r += gridDim.x) {

@@ -513,10 +513,10 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
 //
 // The CUDA-core kernel this replaced (36 FP32 accumulators per thread, 13 shared-memory
 // reads per 36 FMAs) took 1.40 ms per 32 -> 32 layer of 8 x 512 x 512, 11.0 of the 12.6 ms
-// of a training step; this one 0.147 ms (step 2.73 ms). Its MMAs would take 0.04 ms; the
-// copies bound it: a pixel's 8-channel groups lie in different planes, so data arrive in
-// shared memory 16 bytes at a time (with a quarter of the input rows copied it takes 0.115;
-// fewer MMAs, flushes or bias sums change nothing).
+// of a training step; this one 0.104 ms. Its MMAs would take 0.04 ms; the copies bound it:
+// 0.147 ms with NHWC activations (16 bytes at a time), 0.114 by planes with one thread
+// issuing a tile's 24 copies one after another, 0.104 with a lane to each (fewer MMAs,
+// flushes or bias sums change nothing).
 constexpr int kWgStages = 4;
 constexpr int kWgGroup = 4;                          // tiles accumulated in TMEM before a flush
 constexpr int kWgPlane = kHalo * 16;                 // bytes between planes

@@ -37,6 +37,29 @@ def test_several_columns_equal_one(cuda, XN, YN, dz, ZN):
         assert torch.equal(vols[a], vols[b]), (a, b)
 
 
+@pytest.mark.parametrize("YL,ZL", [(104, 5), (100, 3), (101, 4)])
+def test_texture_copy_by_rows(cuda, YL, ZL):
+    """The copy's fill by eight, four and single channels, with row counts that are no multiple of four: an FP16
+    copy blended in 1.8 fixed point against the FP32 copy blended the same, so FP16 rounding of BF16 data (none)."""
+    sc = G.tiny(YL=YL, ZL=ZL, XN=24, YN=20, ZN=7, dx=4.0, dy=4.0, dz=1.0)
+    g = torch.Generator(device=cuda).manual_seed(YL)
+    filt = torch.randn((sc.PN, ZL, YL), device=cuda, generator=g)
+    fast = StagePlans(sc, _lib.HR_FORM_FAST)
+    pairs = torch.empty((sc.PN, ZL, YL), dtype=torch.int32, device=cuda)
+    fast.pack(pairs, filt)
+    vols = {}
+    for v in (11, 14):  # eight slices per thread from the FP16 and the FP32 copy
+        _lib.check(_lib.load().hr_bp_select(fast._bp, v))
+        vols[v] = torch.zeros((sc.YN, sc.XN, sc.ZN), device=cuda)
+        fast.backproject(vols[v], pairs)
+    torch.cuda.synchronize()
+    fast.close()
+    assert int(torch.count_nonzero(vols[14])) > 0
+    # the filter hardware may blend FP16 texels at less precision than FP32 ones: 2^-8 of a neighbour difference
+    d = (vols[11].double() - vols[14].double()).norm() / vols[14].double().norm()
+    assert float(d) < 1e-2, float(d)
+
+
 def test_streamed_ranges_equal_the_whole(cuda, monkeypatch):
     monkeypatch.setenv("HELIXRECON_BP_VARIANT", "21")
     sc = G.Scan(ZL=16, N_2pi=492, pitch=0.9375, rotations=8, XN=300, YN=300, ZN=60, dx=500.0 / 300, dy=500.0 / 300,
