@@ -113,7 +113,7 @@ struct ColView {
 
 template <class PT>
 __device__ __forceinline__ bool col_view(const PT& P, float x, float y, float2 cs, ColView& cv) {
-  const float UU = fmaf(-y, cs.y, -(x * cs.x));
+  const float UU = fmaf(-x, cs.x, -(y * cs.y));
   const float Yr = fmaf(y, cs.x, -(x * cs.y));
   const float t1sq = P.SO2 - Yr * Yr;
   const float temp1 = t1sq * rsqrt_approx(t1sq);
@@ -566,7 +566,7 @@ __device__ __forceinline__ void tex_column(float* __restrict__ vol, const TexRef
     if (mask == 0u) continue;
     const int p = blk.x + q;
     const float2 cs = __ldg(T.trig + p);
-    const float UU = fmaf(-y, cs.y, -(x * cs.x));
+    const float UU = fmaf(-x, cs.x, -(y * cs.y));
     const float Yr = fmaf(y, cs.x, -(x * cs.y));
     const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
     if (!(u1 >= 0.0f && u1 < utop)) continue;  // floor(u1) in [0, YL-2]
@@ -621,8 +621,8 @@ __global__ void __launch_bounds__(kBx* kBy) bp_tex_kernel(float* __restrict__ vo
 // view added exactly 0 there), so both give the same bits.
 //
 // V columns (x, y .. y + V - 1) per thread: what a view costs however many
-// slices hold it (loop, table and trigonometry loads, texture handle and layer,
-// the products with x) is shared by V columns, and 4 V taps are in flight. With
+// slices hold it (loop, table and trigonometry loads, texture handle and layer)
+// is shared by V columns, and 4 V taps are in flight. With
 // V = 1 the kernels ran into instruction issue (56 % of the slots at 55 % of
 // the filter rate on thick slices) before the texture units' rate. V = 4 with 4
 // slices, 64 registers and CTAs of 128 against the best one-column form, chain
@@ -663,13 +663,12 @@ __device__ __forceinline__ void tex_range(float (&res)[V][NZ], const SegCtx<V>& 
   for (int q = q0; q < q1; ++q) {
     const int p = c.blk0 + q;
     const float2 cs = __ldg(c.trig + p);
-    const float xc = c.x * cs.x, xs = c.x * cs.y;
     float K[V], E[V], xt[V];
     bool on[V], any = false;
 #pragma unroll
     for (int h = 0; h < V; ++h) {
-      const float UU = fmaf(-c.y[h], cs.y, -xc);
-      const float Yr = fmaf(c.y[h], cs.x, -xs);
+      const float UU = fmaf(-c.x, cs.x, -(c.y[h] * cs.y));
+      const float Yr = fmaf(c.y[h], cs.x, -(c.x * cs.y));
       const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
       on[h] = u1 >= 0.0f && u1 < c.utop;  // floor(u1) in [0, YL-2]
       any = any || on[h];
@@ -727,7 +726,7 @@ __device__ __forceinline__ void tex_range2(float (&res)[1][NZ], const SegCtx<1>&
     for (int h = 0; h < 2; ++h) {
       const int p = c.blk0 + q + h;
       const float2 cs = __ldg(c.trig + p);
-      const float UU = fmaf(-c.y[0], cs.y, -(c.x * cs.x));
+      const float UU = fmaf(-c.x, cs.x, -(c.y[0] * cs.y));
       const float Yr = fmaf(c.y[0], cs.x, -(c.x * cs.y));
       const float u1 = fmaf(Yr, P.invdYL, P.YLC0);
       onv[h] = u1 >= 0.0f && u1 < c.utop;  // floor(u1) in [0, YL-2]
