@@ -821,6 +821,9 @@ size_t plain_q_smem(const BpParams& P) {
 }
 // Above this the per-CTA weight table would cost too much occupancy (very
 // thick slices: long union windows); the per-update weight kernel runs instead.
+// The limit on a kernel's dynamic shared memory belongs to the kernel, not to a
+// plan: every launch sets it to this most, so that of two plans executed by two
+// threads neither lowers it between the other's setting and launch.
 constexpr size_t kPlainQSmemMax = 96 * 1024;
 
 // Dynamic shared memory of bp_fp64_q_kernel, and the most it may take (two CTAs per SM still fit); above
@@ -843,7 +846,7 @@ int launch_plain(const BpParams& P, float* vol, const float* fp, const ViewTab* 
     grid.x = (P.XN + kTx - 1) / kTx;
     grid.y = (P.YN + kTy - 1) / kTy;
     HR_CUDA_TRY(cudaFuncSetAttribute(bp_plain_q_kernel<kNzPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)qsmem));
+                                     (int)kPlainQSmemMax));
     bp_plain_q_kernel<kNzPlain><<<grid, dim3(kTx, kTy), qsmem, s>>>(vol, fp, views, w, P);
   } else {
     bp_plain_kernel<kNzPlain><<<grid, dim3(kBx, kBy), sizeof(float) * P.N_2pi, s>>>(vol, fp, views, w, P);
@@ -941,7 +944,7 @@ extern "C" int hr_bp_execute(const hr_bp_plan* pl, void* d_vol, const void* d_fp
     if (P.qcap > 0 && qsmem <= kFp64QSmemMax) {
       grid = dim3((P.XN + kDx - 1) / kDx, (P.YN + kDy - 1) / kDy, (P.ZN + kNzFp64Q - 1) / kNzFp64Q);
       HR_CUDA_TRY(cudaFuncSetAttribute(bp_fp64_q_kernel<kNzFp64Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)qsmem));
+                                       (int)kFp64QSmemMax));
       bp_fp64_q_kernel<kNzFp64Q><<<grid, dim3(kDx, kDy), qsmem, s>>>(vol, fp, pl->d_views, pl->d_wd, P);
     } else {
       bp_fp64_kernel<kNzFp64><<<grid, dim3(kBx, kBy), sizeof(double) * P.N_2pi, s>>>(vol, fp, pl->d_views, pl->d_wd,

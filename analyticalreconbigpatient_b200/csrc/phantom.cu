@@ -155,9 +155,11 @@ extern "C" int hr_project_ellipsoids(float* d_proj, int YL, int ZL, int ViewN, d
   HR_REQUIRE(YL > 0 && ZL > 0 && ViewN > 0 && nobj >= 0, "hr_project_ellipsoids: invalid sizes");
   HR_REQUIRE((long long)YL * ZL < (1LL << 31), "hr_project_ellipsoids: YL*ZL too large");
   const size_t smem = sizeof(double) * kObjStride * (size_t)nobj;
-  HR_REQUIRE(smem <= 200 * 1024, "hr_project_ellipsoids: %d objects exceed the shared-memory table", nobj);
+  constexpr size_t most = 200 * 1024;
+  HR_REQUIRE(smem <= most, "hr_project_ellipsoids: %d objects exceed the shared-memory table", nobj);
+  // the limit belongs to the kernel: always the most, so that no other thread's call lowers it before this launch
   if (smem > 48 * 1024)
-    HR_CUDA_TRY(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HR_CUDA_TRY(cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   dim3 grid((YL * ZL + 255) / 256, ViewN < 65535 ? ViewN : 65535);
   project_kernel<<<grid, 256, smem, hr::as_stream(stream)>>>(d_proj, YL, ZL, ViewN, SO, SD, dYA, YLC0, dZL, ZLC0,
                                                              BetaS, dBeta, h, d_obj, nobj);
