@@ -9,7 +9,7 @@
 // |j-m| <= YL-1 through a length-NN circular one. Any circular length
 // N >= 2 YL - 1 gives the same linear convolution, so this filter uses
 // N = 2^ceil(log2(2 YL - 1)) (2048 for YL = 888, the reference pads to 4096),
-// raised to 2048 from 512 on.
+// raised to 2048 from 1024 on, and from 512 on where there are many rows.
 // h is even, so its transform H is real; two real rows a, b are filtered at
 // once as one complex signal a + i b:  ifft(H fft(a + i b)) = (h*a) + i (h*b).
 // The inverse transform is done with the forward one: ifft(Z) =
@@ -23,7 +23,7 @@
 // layout [v][ZL][YL] or in the rebinning's layout [v][YL][ZL]; for the latter
 // the 4 rows of a tile are 16 contiguous bytes per channel.
 //
-// N = 2048 (YL in (128, 1024], the scanners' 888 channels) runs a register-
+// N = 2048 (YL in (256, 1024], the scanners' 888 channels; with many rows from 129 on) runs a register-
 // resident kernel instead: two warps per pair of rows (below), or one, 64 points per lane
 // (N = 64 x 32). Forward: each lane j transforms x[j + 32 m] over m with a
 // 64-point DFT (8 x 8, in registers), multiplies by W_2048^(j c), and the
@@ -844,13 +844,15 @@ int launch_layout(const hr_filter_plan* p, float* out, const float* in, int view
     case 7: return launch_t<7, IN_LAYOUT>(p, out, in, view0, s);
     case 8: return launch_t<8, IN_LAYOUT>(p, out, in, view0, s);
     case 9: return launch_t<9, IN_LAYOUT>(p, out, in, view0, s);
-    case 10: return launch_t<10, IN_LAYOUT>(p, out, in, view0, s);
     case 11: return p->kernel2048 ? fft2k::launch<IN_LAYOUT>(p, out, in, view0, s)
                                   : fft2k::launch2<IN_LAYOUT>(p, out, in, view0, s);
     case 12: return launch_t<12, IN_LAYOUT>(p, out, in, view0, s);
     default: return hr::fail(HR_ERR_UNSUPPORTED, "filter: transform length 2^%d unsupported", p->log2N);
   }
 }
+
+// Rows from which a plan of N = 512 takes the N = 2048 kernel.
+constexpr long long kLongRows = 4096;
 
 }  // namespace
 
@@ -865,11 +867,14 @@ extern "C" int hr_filter_plan_create(hr_filter_plan** plan, int YL, int ZL, int 
   HR_TRY(hr::require_device());
   int log2N = 3;
   while ((1 << log2N) < 2 * YL - 1) ++log2N;
-  // Lengths 512 and 1024 run as 2048 too: the register kernel's longer transforms, pruned to the samples there
-  // are, cost less than the shared-memory kernel's short ones, and their results are nearer to FP64 (32,000
-  // rows of 500 channels 246 -> 126 us, error 5.1e-6 -> 4.4e-6; of 250 channels 138 -> 119 us, 3.1e-6 ->
-  // 2.4e-6; of 100 channels, N = 256, it would be 66 -> 116 us).
-  if (log2N == 9 || log2N == 10) log2N = 11;
+  // Length 1024, and 512 from 4096 rows on, run as 2048 too: the register kernel's longer transforms, pruned to
+  // the samples there are, cost less than the shared-memory kernel's short ones, and their results are nearer to
+  // FP64 (32,000 rows of 500 channels 246 -> 126 us, error 5.1e-6 -> 4.4e-6; of 250 channels 138 -> 119 us,
+  // 3.1e-6 -> 2.4e-6; of 100 channels, N = 256, it would be 66 -> 116 us). Few short rows do not fill the SMs with
+  // either, and the register kernel's larger tables cost more than its transforms save (129 to 256 channels, 16
+  // and 256 rows 8.3 -> 11.3 us, 2048 rows 14.4 with both, 16,000 rows 68 -> 62; from 257 channels on it is no
+  // slower at any count).
+  if (log2N == 10 || (log2N == 9 && (long long)ZL * ViewN >= kLongRows)) log2N = 11;
   const int N = 1 << log2N;
   // Wrapped kernel and its (real) spectrum, in double.
   std::vector<double> hs(N, 0.0);
