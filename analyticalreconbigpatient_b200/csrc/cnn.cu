@@ -472,7 +472,10 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
       r += ny;
       for (int i = 0; i < ny; ++i, ++it) {
         const int acc = it % kSlots;
-        if (!mbar_wait(&tfull[acc], (it / kSlots) & 1, abort_flag, a.err, a.wait_limit)) {
+        const bool waited = mbar_wait(&tfull[acc], (it / kSlots) & 1, abort_flag, a.err, a.wait_limit);
+        // the TMEM instructions below are warp-collective: the whole warp runs them or, where a lane saw an
+        // abort that the others did not, none of it does
+        if (!__all_sync(0xffffffffu, waited)) {
           ok = false;
           break;
         }
