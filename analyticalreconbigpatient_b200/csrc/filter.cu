@@ -126,6 +126,17 @@ __device__ __forceinline__ float2* fft_forward(float2* X, float2* Y, const float
   return X;
 }
 
+// Cosine preweight. For N = 512 its roundings are written out: the two layouts' instances fused the products
+// differently there, and a row's result must not depend on the layout it is read from.
+template <int N>
+__device__ __forceinline__ float preweight(float b, float t, float SO2) {
+  if constexpr (N == 512)
+    return __fdiv_rn(SO2, __fsqrt_rn(__fmaf_rn(-__fmul_rn(__fmul_rn(b, t), b), t,
+                                               __fmul_rn(SO2, __fmaf_rn(b, b, SO2)))));
+  else
+    return SO2 / sqrtf(SO2 * (SO2 + b * b) - b * t * b * t);
+}
+
 template <int LOG2N, int IN_LAYOUT>
 __global__ void __launch_bounds__(kThreads) filter_fft_kernel(float* __restrict__ out, const float* __restrict__ in,
                                                               const float* __restrict__ gH,
@@ -164,8 +175,7 @@ __global__ void __launch_bounds__(kThreads) filter_fft_kernel(float* __restrict_
           float val = 0.0f;
           if (q < nrows && j < YL) {
             const float t = ((float)j - PLC) * dYL;
-            const float wei = SO2 / sqrtf(SO2 * (SO2 + b * b) - b * t * b * t);
-            val = src[j] * wei;
+            val = src[j] * preweight<N>(b, t, SO2);
           }
           dstc[2 * j] = val;
         }
@@ -182,8 +192,7 @@ __global__ void __launch_bounds__(kThreads) filter_fft_kernel(float* __restrict_
           const long long v = r / ZL;
           const float b = ((float)k - ZLC) * dZL;
           const float t = ((float)j - PLC) * dYL;
-          const float wei = SO2 / sqrtf(SO2 * (SO2 + b * b) - b * t * b * t);
-          val = in[((size_t)(view0 + v) * YL + j) * ZL + k] * wei;
+          val = in[((size_t)(view0 + v) * YL + j) * ZL + k] * preweight<N>(b, t, SO2);
         }
         reinterpret_cast<float*>(X + (q >> 1) * N)[2 * j + (q & 1)] = val;
       }
