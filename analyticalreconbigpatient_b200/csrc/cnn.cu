@@ -793,31 +793,34 @@ __global__ void pack_input_kernel(uint16_t* __restrict__ out, const float* __res
 
 // The same input as planes (two groups: 8 channels of which 5 are used, 8 of zeros) for the
 // network itself. A CTA takes 32 padded pixels of one image row and 32 slices: it reads each
-// pixel's 36 consecutive slices together (the volume's fastest axis) and writes rows of pixels.
+// pixel's 36 consecutive slices together (the volume's fastest axis) and writes rows of pixels. Images of more
+// rows than a grid has are walked.
 constexpr int kPackPx = 32, kPackZ = 32;
 __global__ void __launch_bounds__(256) pack_planes_kernel(uint4* __restrict__ out, const float* __restrict__ vol, int XN,
                                                           int YN, int ZN, int z0, int nz, float inv_mu, int Wp) {
   __shared__ float t[kPackPx][kPackZ + 5];
-  const int px0 = blockIdx.x * kPackPx, y = blockIdx.y, s0 = blockIdx.z * kPackZ;
-  for (int i = threadIdx.x; i < kPackPx * (kPackZ + 4); i += 256) {
-    const int p = i / (kPackZ + 4), k = i - p * (kPackZ + 4);
-    const int x = px0 + p - 1, z = min(max(z0 + s0 + k - 2, 0), ZN - 1);
-    if (x >= 0 && x < XN && s0 + k < nz + 4) t[p][k] = vol[((size_t)y * XN + x) * ZN + z];
-  }
-  __syncthreads();
+  const int px0 = blockIdx.x * kPackPx, s0 = blockIdx.z * kPackZ;
   const int p = threadIdx.x & (kPackPx - 1), px = px0 + p, x = px - 1;
-  if (px >= Wp) return;
-  for (int k = threadIdx.x / kPackPx; k < kPackZ && s0 + k < nz; k += 256 / kPackPx) {
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (x >= 0 && x < XN) {
-      float u[5];
-#pragma unroll
-      for (int c = 0; c < 5; ++c) u[c] = t[p][k + c] * inv_mu - 1.0f;
-      w = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], 0.0f), 0u);
+  for (int y = blockIdx.y; y < YN; y += gridDim.y) {
+    for (int i = threadIdx.x; i < kPackPx * (kPackZ + 4); i += 256) {
+      const int q = i / (kPackZ + 4), k = i - q * (kPackZ + 4);
+      const int xq = px0 + q - 1, z = min(max(z0 + s0 + k - 2, 0), ZN - 1);
+      if (xq >= 0 && xq < XN && s0 + k < nz + 4) t[q][k] = vol[((size_t)y * XN + xq) * ZN + z];
     }
-    const size_t o = plane_row(s0 + k, YN, y, 2, 0, Wp) + px;
-    out[o] = w;
-    out[o + Wp] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (int k = threadIdx.x / kPackPx; px < Wp && k < kPackZ && s0 + k < nz; k += 256 / kPackPx) {
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (x >= 0 && x < XN) {
+        float u[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) u[c] = t[p][k + c] * inv_mu - 1.0f;
+        w = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], 0.0f), 0u);
+      }
+      const size_t o = plane_row(s0 + k, YN, y, 2, 0, Wp) + px;
+      out[o] = w;
+      out[o + Wp] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();  // before the next row's values
   }
 }
 
@@ -1220,11 +1223,12 @@ extern "C" int hr_cnn_apply_volume(hr_cnn* n, float* d_out, const float* d_vol, 
   HR_REQUIRE(XN > 0 && YN > 0 && ZN > 0 && chunk > 0 && mu_w > 0.0f, "hr_cnn_apply_volume: invalid sizes");
   cudaStream_t s = hr::as_stream(stream);
   const int Wp = padded_width(XN);
+  constexpr int kGridMax = 65535;  // of a grid's y and z
+  chunk = std::min(chunk, kGridMax * kPackZ);
   HR_TRY(ensure_acts(n, (long long)std::min(chunk, ZN) * YN * Wp));
   for (int z0 = 0; z0 < ZN; z0 += chunk) {
     const int nz = std::min(chunk, ZN - z0);
-    HR_REQUIRE(YN <= 65535 && (nz + kPackZ - 1) / kPackZ <= 65535, "hr_cnn_apply_volume: grid too large");
-    const dim3 grid((Wp + kPackPx - 1) / kPackPx, YN, (nz + kPackZ - 1) / kPackZ);
+    const dim3 grid((Wp + kPackPx - 1) / kPackPx, std::min(YN, kGridMax), (nz + kPackZ - 1) / kPackZ);
     pack_planes_kernel<<<grid, 256, 0, s>>>(n->d_act[0], d_vol, XN, YN, ZN, z0, nz, 1.0f / mu_w, Wp);
     HR_CUDA_TRY(cudaGetLastError());
     HR_TRY(forward_trunk(n, nz, YN, XN, s));
