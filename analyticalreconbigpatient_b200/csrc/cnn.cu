@@ -8,13 +8,21 @@
 //   output : centre slice (FP32, not rounded) + mu_w * L8 channel 0
 //
 // Inside the network activations and gradients are stored by planes: [B][H][C / 8][Wp][8]
-// BF16, a row of 16-byte pixel chunks per 8 channels with Wp = 128 ceil(W / 128) + 2 chunks,
-// one zero chunk before the image's first pixel and zeros after its last, so that a tile's
-// halo row is 130 contiguous chunks wherever it lies (rows above and below the image come
-// from a zero row). One untiled bulk copy brings such a row into shared memory, and an
-// epilogue's stores are contiguous over the warp. (With NHWC activations the same rows were
-// TMA boxes of 8 channels x 130 pixels, 16 bytes at a time, and bounded the kernels.) Every
-// epilogue writes its rows' zero chunks too, so nothing depends on what a buffer held.
+// BF16, a row of 16-byte pixel chunks per 8 channels with Wp = W + 2 chunks, a zero chunk
+// before the image's first pixel and one after its last, so that a tile's halo row is at most
+// 130 contiguous chunks wherever it lies (rows above and below the image come from a zero
+// row). One untiled bulk copy brings such a row into shared memory, and an epilogue's stores
+// are contiguous over the warp. (With NHWC activations the same rows were TMA boxes of 8
+// channels x 130 pixels, 16 bytes at a time, and bounded the kernels.) Every epilogue writes
+// its rows' two zero chunks too, and a row's last tile takes no more than the row has, so
+// nothing depends on what a buffer held. (Rows padded to whole tiles would need no short
+// tile, but up to eight times the memory for narrow images, twice for W = 129.)
+//
+// Buffers: inference alternates between two activations (layer k reads one and writes the
+// other) and keeps the input: 80 channels per pixel instead of the 304 of all layers and
+// gradients. A training step needs every layer's output; its gradients alternate between a
+// buffer and the last layer's input, of which the gradient's first step is the last use (288
+// channels per pixel). Both are kept from call to call.
 //
 // Convolutions run as implicit GEMMs on the 5th-generation tensor cores: one
 // tile is 128 output pixels of one image row (M = 128, TMEM lanes) by COUT
@@ -179,7 +187,7 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 
 // Chunks of a padded row, and the chunk offset of channel group c of image row (b, y) (G groups).
-__host__ __device__ constexpr int padded_width(int W) { return (W + kTileM - 1) / kTileM * kTileM + 2; }
+__host__ __device__ constexpr int padded_width(int W) { return W + 2; }
 __device__ __forceinline__ size_t plane_row(int b, int H, int y, int G, int c, int Wp) {
   return (((size_t)b * H + y) * G + c) * Wp;
 }
@@ -260,16 +268,21 @@ struct ConvArgs {
 template <int COUT, int EPI>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v)[COUT], const float* bias_s, int b,
                                               int y, int x, int lane) {
-  const bool valid = x < a.W;  // pixels beyond the image are stored as zeros
+  const bool valid = x < a.W;  // a tile's pixels beyond the image hold nothing
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   const size_t row = plane_row(b, a.H, y, COUT / 8, 0, a.Wp);
-  if constexpr (EPI != EPI_RESID && EPI != EPI_RAW) {  // the zero chunks before the first and after the last tile pixel
-    if (x == 0 || x == a.Wp - 3) {
+  if constexpr (EPI != EPI_RESID && EPI != EPI_RAW) {  // the zero chunks before the first and after the last pixel
+    if (x == 0) {
 #pragma unroll
-      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + (x == 0 ? 0 : a.Wp - 1)] = zero;
+      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp] = zero;
+    }
+    if (x == a.W - 1) {
+#pragma unroll
+      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + a.Wp - 1] = zero;
     }
   }
   if constexpr (EPI == EPI_RELU) {
+    if (!valid) return;
     uint4* o = a.out + row + x + 1;
 #pragma unroll
     for (int c = 0; c < COUT / 8; ++c) {
@@ -279,16 +292,15 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
       float u[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) u[j] = fmaxf(v[8 * c + j] + bias[j], 0.0f);
-      o[(size_t)c * a.Wp] = valid ? make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]),
-                                               pack2(u[6], u[7]))
-                                  : zero;
+      o[(size_t)c * a.Wp] = make_uint4(pack2(u[0], u[1]), pack2(u[2], u[3]), pack2(u[4], u[5]), pack2(u[6], u[7]));
     }
   } else if constexpr (EPI == EPI_MASK) {
+    if (!valid) return;
     const uint4* m = a.mask + row + x + 1;
     uint4* o = a.out + row + x + 1;
 #pragma unroll
     for (int c = 0; c < COUT / 8; ++c) {
-      const uint4 mv = __ldg(m + (size_t)c * a.Wp);  // zero beyond the image: masks those pixels too
+      const uint4 mv = __ldg(m + (size_t)c * a.Wp);
       const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
       float u[8];
 #pragma unroll
@@ -318,7 +330,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, const float (&v
     }
     if constexpr (EPI == EPI_LOSS) {
 #pragma unroll
-      for (int c = 0; c < COUT / 8; ++c) a.out[row + (size_t)c * a.Wp + x + 1] = c == 0 ? g0 : zero;
+      for (int c = 0; c < COUT / 8; ++c)
+        if (valid) a.out[row + (size_t)c * a.Wp + x + 1] = c == 0 ? g0 : zero;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
       if (lane == 0 && e2 != 0.0f) atomicAdd(a.loss, e2);
@@ -332,7 +345,6 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
   constexpr int kRow = G * kPlane;           // bytes of one input row (130 pixels)
   constexpr int kWBytes = 9 * CIN * COUT * 2;
   constexpr int kKSteps = 3 * CIN / 16;      // per input row: horizontal taps x 16-channel steps
-  constexpr uint32_t kTxBytes = G * kBox;
   static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "unsupported channel counts");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -389,6 +401,9 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
   if (warp == 0) {
     // ---- producer: input rows of each piece into the ring, G halo rows each ------------------
     if (lane == 0) {
+      // a row's last strip may be short: what lies behind its chunks in the ring feeds only accumulator rows
+      // of pixels beyond the image, which the epilogue leaves out
+      const uint32_t bytes = (uint32_t)(min(a.W - seg * kTileM, kTileM) + 2) * 16;
       int h = 0;  // input rows loaded by this CTA
       int last_h[kRing];
       for (int s = 0; s < kRing; ++s) last_h[s] = -1;
@@ -405,12 +420,12 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
           }
           if (h == a.stall_row) continue;  // test hook: this row's slot is never filled
           last_h[s] = h;
-          mbar_expect_tx(&full[s], kTxBytes);
+          mbar_expect_tx(&full[s], G * bytes);
           const int y = y0 - 1 + j;
           const bool in = y >= 0 && y < a.H;
           const uint4* src = in ? a.in + plane_row(b, a.H, y, G, 0, a.Wp) + seg * kTileM : a.zero;
           for (int g = 0; g < G; ++g)
-            bulk_load(smem_a + s * kRow + g * kPlane, src + (in ? (size_t)g * a.Wp : 0), kBox, &full[s]);
+            bulk_load(smem_a + s * kRow + g * kPlane, src + (in ? (size_t)g * a.Wp : 0), bytes, &full[s]);
         }
       }
       // every issued copy lands before the CTA exits (after an abort nobody consumes them)
@@ -530,7 +545,7 @@ constexpr int kWgThreads = 32 * (kWgWorkers + 2);
 constexpr int kWgTmemCols = 512;
 constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256;
 
-template <int CIN, int COUT>
+template <int CIN, int COUT, bool RAGGED>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __restrict__ X,
                                                                  const uint4* __restrict__ Gr,
                                                                  const uint4* __restrict__ zero, int B, int H, int W,
@@ -580,9 +595,14 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
   const uint32_t smem0 = smem_u32(wg_smem);
 
   const int Wp = padded_width(W);
-  const uint32_t nseg = (uint32_t)(Wp - 2) / kTileM, npair = (uint32_t)(H + 1) / 2;
+  const uint32_t nseg = (uint32_t)(W + kTileM - 1) / kTileM, npair = (uint32_t)(H + 1) / 2;
   const uint32_t tiles = (uint32_t)B * npair * nseg;                                 // < 2^31, checked at launch
   const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);             // this CTA's (grid <= tiles)
+  // pixels of this CTA's i-th tile: with ragged widths a row's last strip is short, and the sums stop with it
+  auto tile_pixels = [&](int i) {
+    if constexpr (!RAGGED) return kTileM;
+    return min(W - (int)((blockIdx.x + (uint32_t)i * gridDim.x) % nseg) * kTileM, kTileM);
+  };
 
   if (warp < kWgWorkers) {
     // ---- bias sums and flushes -------------------------------------------------------------------
@@ -622,6 +642,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
     const int gc = tid % GC, gp = tid / GC;
     for (int j = 0; j < n && ok; ++j) {
       const int s = j % kWgStages;
+      const int np = tile_pixels(j);
       const bool waited =
           lane != 0 || mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
       if (!__all_sync(0xffffffffu, waited)) {
@@ -633,7 +654,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       for (int row = 0; row < 2; ++row)
 #pragma unroll
         for (int px = 0; px < kTileM; px += 32 * kWgWorkers / GC) {
-          const uint4 w = *reinterpret_cast<const uint4*>(st + (row * GC + gc) * kWgPlane + (gp + px) * 16);
+          uint4 w = *reinterpret_cast<const uint4*>(st + (row * GC + gc) * kWgPlane + (gp + px) * 16);
+          if (RAGGED && gp + px >= np) w = make_uint4(0u, 0u, 0u, 0u);
           const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -673,6 +695,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       for (int j = 0; j < n && ok; ++j) {
         const int s = j % kWgStages, grp = j / kWgGroup, b = grp & 1;
         const bool first = j % kWgGroup == 0;
+        const int np = tile_pixels(j);
         if (first && grp >= 2)
           ok = mbar_wait(&tempty[b], (uint32_t)((grp >> 1) - 1) & 1, abort_flag, err, kWaitLimit);
         if (ok) ok = mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
@@ -683,11 +706,18 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
         // an offset of 16 bytes is one unit of a descriptor's address
         const uint64_t ad = desc_noswz(xa, 128, kWgPlane), bd = desc_noswz(ga, 128, kWgPlane);
         const uint32_t acc = tmem + b * 3 * kN;
+        if (!RAGGED || np == kTileM) {
 #pragma unroll
-        for (int ks = 0; ks < kTileM / 16; ++ks)
+          for (int ks = 0; ks < kTileM / 16; ++ks)
 #pragma unroll
-          for (int dx = 0; dx < 3; ++dx)
-            umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
+            for (int dx = 0; dx < 3; ++dx)
+              umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
+        } else {
+          for (int ks = 0; ks < (np + 15) / 16; ++ks)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+              umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
+        }
         umma_commit(&empty[s]);
         if (j % kWgGroup == kWgGroup - 1 || j == n - 1) umma_commit(&tfull[b]);
       }
@@ -709,14 +739,25 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       if (!__all_sync(0xffffffffu, free)) break;
       const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / nseg;
       const int x0 = (int)(t - by * nseg) * kTileM, b = (int)(by / npair), y = 2 * (int)(by - (uint32_t)b * npair);
-      if (lane == 0) mbar_expect_tx(&full[s], 4 * XC * kBox + 2 * GC * kTileM * 16);
+      const int np = RAGGED ? min(W - x0, kTileM) : kTileM;
+      const uint32_t d = dst + (uint32_t)s * kWgStage;
+      if (RAGGED && np % 16 != 0) {  // zeros, in both operands, for the pixels that the last MMA of a short strip has too many
+        if (lane < 4 * XC + 2 * GC)
+          for (int k = np; k < ((np + 15) & ~15); ++k)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(d + (uint32_t)(xrow ? k + 2 : k) * 16),
+                         "r"(0)
+                         : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+      }
+      if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(4 * XC * (np + 2) + 2 * GC * np) * 16);
       __syncwarp();
       if (lane < 4 * XC + 2 * GC) {
         const int yy = xrow ? y + row - 1 : y + row;
         const uint4* src = zero;
         if (yy >= 0 && yy < H)
           src = xrow ? X + plane_row(b, H, yy, XC, c, Wp) + x0 : Gr + plane_row(b, H, yy, GC, c, Wp) + x0 + 1;
-        bulk_load(dst + (uint32_t)s * kWgStage, src, xrow ? kBox : kTileM * 16, &full[s]);
+        bulk_load(d, src, (uint32_t)(xrow ? np + 2 : np) * 16, &full[s]);
       }
       issued = i + 1;
     }
@@ -923,17 +964,24 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
   return launch_dependent(conv_tc_kernel<CIN, COUT, EPI>, (unsigned)grid, kThreads, smem, s, a);
 }
 
-template <int CIN, int COUT>
-int launch_wgrad(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
-                 int* err, cudaStream_t s) {
+template <int CIN, int COUT, bool RAGGED>
+int launch_wgrad_of(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
+                    int* err, cudaStream_t s) {
   const long long tiles = (long long)B * ((H + 1) / 2) * ((W + kTileM - 1) / kTileM);
   const long long grid = std::min<long long>(tiles, hr::sm_count());
   if (grid <= 0) return HR_OK;
   HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
-  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kWgSmem));
-  return launch_dependent(wgrad_tc_kernel<CIN, COUT>, (unsigned)grid, kWgThreads, kWgSmem, s, X, Gr, zero, B, H, W,
-                          dW, db, err);
+  return launch_dependent(wgrad_tc_kernel<CIN, COUT, RAGGED>, (unsigned)grid, kWgThreads, kWgSmem, s, X, Gr, zero, B,
+                          H, W, dW, db, err);
+}
+
+template <int CIN, int COUT>
+int launch_wgrad(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
+                 int* err, cudaStream_t s) {
+  if (W % kTileM) return launch_wgrad_of<CIN, COUT, true>(X, Gr, zero, B, H, W, dW, db, err, s);
+  return launch_wgrad_of<CIN, COUT, false>(X, Gr, zero, B, H, W, dW, db, err, s);
 }
 
 }  // namespace
@@ -943,10 +991,12 @@ struct hr_cnn {
   size_t woff[kLayers], boff[kLayers], nparam = 0;
   float *d_p = nullptr, *d_g = nullptr, *d_m = nullptr, *d_v = nullptr;
   uint16_t *d_wf[kLayers] = {}, *d_wb[kLayers] = {};  // BF16 operand images (forward, backward)
-  // activation / gradient planes for up to cap_pix padded pixels (B * H * padded_width(W))
-  long long cap_pix = 0;
-  uint4* d_act[kLayers] = {};  // [0]: input (16 ch), [k]: output of layer k (32 ch), k = 1..7
-  uint4 *d_g0 = nullptr, *d_g1 = nullptr;  // ping-pong gradients (32 ch)
+  // activation planes for up to cap_pix padded pixels (B * H * padded_width(W)); those only training needs, [3]
+  // to [7], d_gout and d_g1, for up to cap_train
+  long long cap_pix = 0, cap_train = 0;
+  uint4* d_act[kLayers] = {};  // [0]: input (16 ch), [k]: output of layer k (32 ch), k = 1..7; inference uses [1], [2]
+  uint4* d_gout = nullptr;     // gradient at the last layer's output (16 ch)
+  uint4* d_g1 = nullptr;       // gradients (32 ch), in turn with d_act[7]
   uint4* d_zero = nullptr;     // kHalo zero chunks: the rows above and below an image
   float* d_loss = nullptr;
   int* d_err = nullptr;
@@ -958,20 +1008,32 @@ struct hr_cnn {
 
 namespace {
 
-void cnn_free_acts(hr_cnn* n) {
-  for (auto& p : n->d_act) {
-    cudaFree(p);
-    p = nullptr;
+constexpr int kInferActs = 3;  // activations that inference uses too
+
+void cnn_free_acts(hr_cnn* n, int l0, int l1) {
+  for (int l = l0; l < l1; ++l) {
+    cudaFree(n->d_act[l]);
+    n->d_act[l] = nullptr;
   }
-  cudaFree(n->d_g0);
-  cudaFree(n->d_g1);
-  n->d_g0 = n->d_g1 = nullptr;
+}
+
+void cnn_free_infer(hr_cnn* n) {
+  cnn_free_acts(n, 0, kInferActs);
   n->cap_pix = 0;
+}
+
+void cnn_free_train(hr_cnn* n) {
+  cnn_free_acts(n, kInferActs, kLayers);
+  cudaFree(n->d_gout);
+  cudaFree(n->d_g1);
+  n->d_gout = n->d_g1 = nullptr;
+  n->cap_train = 0;
 }
 
 void cnn_destroy(hr_cnn* n) {
   if (!n) return;
-  cnn_free_acts(n);
+  cnn_free_infer(n);
+  cnn_free_train(n);
   cudaFree(n->d_p);
   cudaFree(n->d_g);
   cudaFree(n->d_m);
@@ -986,14 +1048,23 @@ void cnn_destroy(hr_cnn* n) {
   delete n;
 }
 
-int ensure_acts(hr_cnn* n, long long pix) {
+// Buffers for `pix` padded pixels.
+int ensure_infer(hr_cnn* n, long long pix) {
   if (pix <= n->cap_pix) return HR_OK;
-  cnn_free_acts(n);
-  HR_CUDA_TRY(cudaMalloc(&n->d_act[0], (size_t)pix * 16 * 2));
-  for (int l = 1; l < kLayers; ++l) HR_CUDA_TRY(cudaMalloc(&n->d_act[l], (size_t)pix * 32 * 2));
-  HR_CUDA_TRY(cudaMalloc(&n->d_g0, (size_t)pix * 32 * 2));
-  HR_CUDA_TRY(cudaMalloc(&n->d_g1, (size_t)pix * 32 * 2));
+  cnn_free_infer(n);
+  for (int l = 0; l < kInferActs; ++l) HR_CUDA_TRY(cudaMalloc(&n->d_act[l], (size_t)pix * (l == 0 ? 16 : 32) * 2));
   n->cap_pix = pix;
+  return HR_OK;
+}
+
+int ensure_train(hr_cnn* n, long long pix) {
+  HR_TRY(ensure_infer(n, pix));
+  if (pix <= n->cap_train) return HR_OK;
+  cnn_free_train(n);
+  for (int l = kInferActs; l < kLayers; ++l) HR_CUDA_TRY(cudaMalloc(&n->d_act[l], (size_t)pix * 32 * 2));
+  HR_CUDA_TRY(cudaMalloc(&n->d_gout, (size_t)pix * 16 * 2));
+  HR_CUDA_TRY(cudaMalloc(&n->d_g1, (size_t)pix * 32 * 2));
+  n->cap_train = pix;
   return HR_OK;
 }
 
@@ -1005,11 +1076,10 @@ int refresh_images(hr_cnn* n, cudaStream_t s) {
   return HR_OK;
 }
 
-// A caller's NHWC input into the planes d_act[0].
+// A caller's NHWC input into the planes d_act[0] (whose buffer is there).
 int load_input(hr_cnn* n, const uint16_t* d_x, int B, int H, int W, cudaStream_t s) {
   const long long rows = (long long)B * H;
   const int Wp = padded_width(W);
-  HR_TRY(ensure_acts(n, rows * Wp));
   const long long blocks = std::min<long long>((rows * Wp + 255) / 256, 16LL * hr::sm_count());
   if (((uintptr_t)d_x & 15) == 0)
     nhwc_to_planes_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
@@ -1032,14 +1102,17 @@ ConvArgs base_args(const hr_cnn* n, int B, int H, int W) {
   return a;
 }
 
-// Layers 1..7 (ReLU) from d_act[0] into d_act[1..7].
-int forward_trunk(hr_cnn* n, int B, int H, int W, cudaStream_t s) {
+// Where layer l's output (l = 1..7) is held: by inference in d_act[1] and d_act[2] in turn.
+int act_index(int l, bool train) { return train || l == 0 ? l : 1 + (l - 1) % 2; }
+
+// Layers 1..7 (ReLU) from d_act[0], into d_act[1..7] for training.
+int forward_trunk(hr_cnn* n, int B, int H, int W, bool train, cudaStream_t s) {
   for (int l = 0; l < kLayers - 1; ++l) {
     ConvArgs a = base_args(n, B, H, W);
-    a.in = n->d_act[l];
+    a.in = n->d_act[act_index(l, train)];
     a.wimg = n->d_wf[l];
     a.bias = n->d_p + n->boff[l];
-    a.out = n->d_act[l + 1];
+    a.out = n->d_act[act_index(l + 1, train)];
     if (l == 0)
       HR_TRY((launch_conv<16, 32, EPI_RELU>(a, s)));
     else
@@ -1126,16 +1199,17 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
   HR_REQUIRE(((uintptr_t)d_x & 15) == 0, "hr_cnn_train_step: input must be 16-byte aligned");
   cudaStream_t s = hr::as_stream(stream);
   const long long pix = (long long)B * H * W;
+  HR_TRY(ensure_train(n, (long long)B * H * padded_width(W)));
   HR_TRY(load_input(n, d_x, B, H, W, s));
   HR_CUDA_TRY(cudaMemsetAsync(n->d_loss, 0, sizeof(float), s));
   HR_CUDA_TRY(cudaMemsetAsync(n->d_g, 0, n->nparam * sizeof(float), s));
-  HR_TRY(forward_trunk(n, B, H, W, s));
+  HR_TRY(forward_trunk(n, B, H, W, true, s));
   // L8 with the fused residual, loss and output gradient (16 channels, channel 0 used)
   ConvArgs a = base_args(n, B, H, W);
   a.in = n->d_act[7];
   a.wimg = n->d_wf[7];
   a.bias = n->d_p + n->boff[7];
-  a.out = n->d_g0;
+  a.out = n->d_gout;
   a.base = d_base;
   a.target = d_target;
   a.sb = (long long)H * W;
@@ -1145,7 +1219,7 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
   a.loss = n->d_loss;
   HR_TRY((launch_conv<32, 16, EPI_LOSS>(a, s)));
   // backward: G_k (gradient at layer k's output) -> dW_k, and G_{k-1} masked by act_{k-1} > 0
-  uint4* g = n->d_g0;
+  uint4* g = n->d_gout;
   uint4* gn = n->d_g1;
   for (int l = kLayers - 1; l >= 0; --l) {
     const int ci = kCin[l], co = kCout[l];
@@ -1167,7 +1241,8 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
       HR_TRY((launch_conv<16, 32, EPI_MASK>(b, s)));
     else
       HR_TRY((launch_conv<32, 32, EPI_MASK>(b, s)));
-    std::swap(g, gn);
+    g = gn;
+    gn = g == n->d_g1 ? n->d_act[kLayers - 1] : n->d_g1;  // act_7 has served as mask and for dW_8
   }
   if (lr > 0.0f) {
     ++n->step;
@@ -1189,9 +1264,9 @@ extern "C" int hr_cnn_train_step(hr_cnn* n, const uint16_t* d_x, const float* d_
 // Layers 1..8 from the input planes in d_act[0], with the residual epilogue.
 static int forward_residual(hr_cnn* n, float* d_out, const float* d_base, long long sb, long long sp, int B, int H,
                             int W, float mu_w, cudaStream_t s) {
-  HR_TRY(forward_trunk(n, B, H, W, s));
+  HR_TRY(forward_trunk(n, B, H, W, false, s));
   ConvArgs a = base_args(n, B, H, W);
-  a.in = n->d_act[7];
+  a.in = n->d_act[act_index(7, false)];
   a.wimg = n->d_wf[7];
   a.bias = n->d_p + n->boff[7];
   a.base = d_base;
@@ -1209,6 +1284,7 @@ extern "C" int hr_cnn_forward(hr_cnn* n, float* d_out, const uint16_t* d_x, cons
   HR_REQUIRE(n != nullptr && d_out != nullptr && d_x != nullptr && d_base != nullptr, "hr_cnn_forward: NULL argument");
   HR_REQUIRE(B > 0 && H > 0 && W > 0 && mu_w > 0.0f, "hr_cnn_forward: invalid sizes");
   cudaStream_t s = hr::as_stream(stream);
+  HR_TRY(ensure_infer(n, (long long)B * H * padded_width(W)));
   HR_TRY(load_input(n, d_x, B, H, W, s));
   return forward_residual(n, d_out, d_base, sb, sp, B, H, W, mu_w, s);
 }
@@ -1225,18 +1301,18 @@ extern "C" int hr_cnn_apply_volume(hr_cnn* n, float* d_out, const float* d_vol, 
   const int Wp = padded_width(XN);
   constexpr int kGridMax = 65535;  // of a grid's y and z
   chunk = std::min(chunk, kGridMax * kPackZ);
-  HR_TRY(ensure_acts(n, (long long)std::min(chunk, ZN) * YN * Wp));
+  HR_TRY(ensure_infer(n, (long long)std::min(chunk, ZN) * YN * Wp));
   for (int z0 = 0; z0 < ZN; z0 += chunk) {
     const int nz = std::min(chunk, ZN - z0);
     const dim3 grid((Wp + kPackPx - 1) / kPackPx, std::min(YN, kGridMax), (nz + kPackZ - 1) / kPackZ);
     pack_planes_kernel<<<grid, 256, 0, s>>>(n->d_act[0], d_vol, XN, YN, ZN, z0, nz, 1.0f / mu_w, Wp);
     HR_CUDA_TRY(cudaGetLastError());
-    HR_TRY(forward_trunk(n, nz, YN, XN, s));
+    HR_TRY(forward_trunk(n, nz, YN, XN, false, s));
     ConvArgs a = base_args(n, nz, YN, XN);
-    a.in = n->d_act[7];
+    a.in = n->d_act[act_index(7, false)];
     a.wimg = n->d_wf[7];
     a.bias = n->d_p + n->boff[7];
-    a.pred = reinterpret_cast<float*>(n->d_g0);  // free between training steps
+    a.pred = reinterpret_cast<float*>(n->d_act[act_index(6, false)]);  // the activation layer 8 does not read
     HR_TRY((launch_conv<32, 16, EPI_RAW>(a, s)));
     const long long px = (long long)XN * YN;
     const dim3 rgrid((unsigned)((px + 31) / 32), (nz + 31) / 32);

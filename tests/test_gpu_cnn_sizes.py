@@ -1,4 +1,5 @@
-"""The correction network at sizes its launches and buffers could limit: images of more rows than a grid holds."""
+"""The correction network at sizes its launches and buffers could limit: images of more rows than a grid holds, and the
+device memory a network takes for widths around its 128-pixel tiles."""
 import pytest
 import torch
 
@@ -23,3 +24,37 @@ def test_volume_of_more_rows_than_a_grid(cuda):
     net.close()
     assert torch.equal(out.permute(2, 0, 1), ref)
     assert float((out - vol).abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("W", [16, 64, 130])
+@pytest.mark.parametrize("call", ["forward", "train_step", "apply_volume"])
+def test_buffers_are_no_larger_than_unpadded_planes(cuda, call, W):
+    """At most 304 channels of two bytes per pixel, the input's 16, seven activations and two gradients of 32, in
+    rows of two pixels more than the image's: narrow images must not be padded to whole tiles in memory."""
+    H = (1 << 22) // W
+    base = torch.full((1, H, W), MU_WATER, device=cuda)
+    vol = base.reshape(H, W, 1).contiguous()
+    out = torch.empty_like(vol)
+    x = torch.zeros((1, H, W, 16), dtype=torch.int16, device=cuda)
+    small = L.Corrector(seed=1)  # the kernels' own first-launch memory is not the network's
+    for n in (1, 2):
+        small.forward(x[:, :n].contiguous(), base[:, :n].contiguous())
+        small.train_step(x[:, :n].contiguous(), base[:, :n].contiguous(), base[:, :n].contiguous(), lr=0.0)
+        small.apply_volume(vol[:n].contiguous())
+    small.close()
+    net = L.Corrector(seed=1)
+    pred = torch.empty_like(base)  # what forward() allocates for its result comes from torch's pool
+    del pred
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    if call == "forward":
+        net.forward(x, base)
+    elif call == "train_step":
+        net.train_step(x, base, base, lr=0.0)
+    else:
+        net.apply_volume(vol, out)
+    torch.cuda.synchronize()
+    used = free - torch.cuda.mem_get_info()[0]
+    net.check()
+    net.close()
+    assert 0 < used <= 304 * 2 * H * (W + 2) + (32 << 20), used / (H * W)
