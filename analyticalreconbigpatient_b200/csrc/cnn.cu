@@ -887,8 +887,8 @@ __global__ void __launch_bounds__(256) add_residual_kernel(float* __restrict__ o
     }
 }
 
-// A caller's NHWC input [rows][W][16] as planes (ALIGNED: it starts on a 16-byte boundary).
-template <bool ALIGNED>
+// A caller's NHWC input [rows][W][16] as planes; ALIGN: the boundary it starts on, 16, 2 or 1 bytes.
+template <int ALIGN>
 __global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* __restrict__ in, long long rows, int W,
                                       int Wp) {
   const long long total = rows * Wp;
@@ -901,11 +901,18 @@ __global__ void nhwc_to_planes_kernel(uint4* __restrict__ out, const uint16_t* _
       uint4 w = make_uint4(0u, 0u, 0u, 0u);
       if (x >= 0 && x < W) {
         const uint16_t* src = in + (r * W + x) * 16 + c * 8;
-        if constexpr (ALIGNED)
+        auto at = [&](int k) -> uint32_t {
+          if constexpr (ALIGN == 1) {
+            const uint8_t* b = reinterpret_cast<const uint8_t*>(src) + 2 * k;
+            return b[0] | (uint32_t)b[1] << 8;
+          } else {
+            return src[k];
+          }
+        };
+        if constexpr (ALIGN == 16)
           w = __ldg(reinterpret_cast<const uint4*>(src));
         else
-          w = make_uint4(src[0] | (uint32_t)src[1] << 16, src[2] | (uint32_t)src[3] << 16,
-                         src[4] | (uint32_t)src[5] << 16, src[6] | (uint32_t)src[7] << 16);
+          w = make_uint4(at(0) | at(1) << 16, at(2) | at(3) << 16, at(4) | at(5) << 16, at(6) | at(7) << 16);
       }
       out[(r * 2 + c) * Wp + px] = w;
     }
@@ -1082,9 +1089,11 @@ int load_input(hr_cnn* n, const uint16_t* d_x, int B, int H, int W, cudaStream_t
   const int Wp = padded_width(W);
   const long long blocks = std::min<long long>((rows * Wp + 255) / 256, 16LL * hr::sm_count());
   if (((uintptr_t)d_x & 15) == 0)
-    nhwc_to_planes_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
+    nhwc_to_planes_kernel<16><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
+  else if (((uintptr_t)d_x & 1) == 0)
+    nhwc_to_planes_kernel<2><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
   else
-    nhwc_to_planes_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
+    nhwc_to_planes_kernel<1><<<(unsigned)blocks, 256, 0, s>>>(n->d_act[0], d_x, rows, W, Wp);
   HR_CUDA_TRY(cudaGetLastError());
   return HR_OK;
 }

@@ -1,9 +1,9 @@
 """The correction network at sizes its launches and buffers could limit: images of more rows than a grid holds, and the
-device memory a network takes for widths around its 128-pixel tiles."""
+device memory a network takes for widths around its 128-pixel tiles, inputs on any byte boundary."""
 import pytest
 import torch
 
-from analyticalreconbigpatient_b200 import learned as L
+from analyticalreconbigpatient_b200 import _lib, learned as L
 from analyticalreconbigpatient_b200.geometry import MU_WATER
 from oracle import cnn_oracle as C
 
@@ -58,3 +58,22 @@ def test_buffers_are_no_larger_than_unpadded_planes(cuda, call, W):
     net.check()
     net.close()
     assert 0 < used <= 304 * 2 * H * (W + 2) + (32 << 20), used / (H * W)
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3, 8])
+def test_input_on_any_byte_boundary(cuda, shift):
+    """forward() takes an input that starts anywhere, as the copy it is brought in by may."""
+    B, H, W = 2, 3, 131
+    g = torch.Generator(device=cuda).manual_seed(shift)
+    x = (0.3 * torch.randn((B, H, W, 16), device=cuda, generator=g)).to(torch.bfloat16).view(torch.int16)
+    base = torch.full((B, H, W), MU_WATER, device=cuda)
+    raw = torch.zeros(x.numel() * 2 + 16, dtype=torch.uint8, device=cuda)
+    raw[shift:shift + x.numel() * 2] = x.reshape(-1).view(torch.uint8)
+    net = L.Corrector(C.init_params(3, zero_last=False))
+    ref = net.forward(x, base)
+    out = torch.full_like(base, float("nan"))
+    _lib.check(_lib.load().hr_cnn_forward(net._net, out.data_ptr(), raw.data_ptr() + shift, base.data_ptr(), H * W, 1,
+                                          B, H, W, MU_WATER, torch.cuda.current_stream().cuda_stream))
+    net.check()
+    net.close()
+    assert torch.equal(out, ref)
