@@ -981,7 +981,7 @@ extern "C" int hr_bp_select(hr_bp_plan* pl, int variant) {
 
 extern "C" int hr_bp_describe(const hr_bp_plan* pl, char* buf, int len) {
   HR_REQUIRE(pl != nullptr, "hr_bp_describe: NULL plan");
-  if (pl->form == HR_FORM_FAST) return hr::bp_fast_describe(pl->fast, buf, len);
+  if (pl->form == HR_FORM_FAST) return hr::bp_fast_describe(pl->fast, pl->fg, buf, len);
   if (buf && len > 0)
     snprintf(buf, (size_t)len, "%s slices_per_thread=%d tile=%dx%d%s", pl->form == HR_FORM_FP64 ? "fp64" : "plain",
              pl->form == HR_FORM_FP64 ? kNzFp64 : kNzPlain, kBx, kBy,

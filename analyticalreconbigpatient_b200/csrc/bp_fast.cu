@@ -785,7 +785,7 @@ __device__ __forceinline__ void tex_dispatch(float (&res)[V][NZ], const SegCtx<V
     tex_dispatch<NZ, V, VIEWS, MA + 1, MA + 1>(res, c, P, sg);
 }
 
-// V columns (xi, yi), (xi, yi + 1) of z block b with the segmented view loop (segments in T.seg).
+// V columns (xi, yi) .. (xi, yi + V - 1) of z block b with the segmented view loop (segments in T.seg).
 template <int NZ, int V = 1, int VIEWS = 1>
 __device__ __forceinline__ void tex_seg_column(float* __restrict__ vol, const TexRef& X, const ZTabs& T,
                                                const FastParams& P, int xi, int yi, int b) {
@@ -1311,19 +1311,47 @@ static void launch_tex_seg(const BpFastTables& t, const BpFast& f, const FastPar
     bp_tex_seg_kernel<NZ, V, VIEWS><<<grid, seg_threads(V), 0, s>>>(vol, texref(f), ztabs(t, f), P, b_first);
 }
 
+// CTAs per SM of a variant's several-column kernel.
+template <class K>
+static int seg_cols_per_sm(K kern) {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, seg_threads(kSegCols), 0) != cudaSuccess) n = 1;
+  return std::max(n, 1);
+}
+static int seg_cols_per_sm(int v) {
+  static const int n18 = seg_cols_per_sm(bp_tex_seg_kernel<8, kSegCols, 1>);
+  static const int n19 = seg_cols_per_sm(bp_tex_seg_kernel<4, kSegCols, 1>);
+  static const int n21 = seg_cols_per_sm(bp_tex_seg_occ_kernel<4, kSegCols, 1>);
+  return v == 18 ? n18 : v == 19 ? n19 : n21;
+}
+
 // Whether a launch over z blocks [b_first, b_first + b_count) has the CTAs for kSegCols columns per thread: two
 // rounds of them, blocks without views not counted. Fewer leave SMs idle at the end, and beside another kernel (a
 // slab's or chunk's filter) one round of long CTAs keeps that kernel out until it ends. Measured, several columns
 // against two views: 512 x 512 x 16 (1.7 rounds) 4.80 / 5.00 ms, 301 x 301 x 40 (1.6) 4.64 / 4.71, 256 x 256 x 24
 // (0.6) 1.82 / 1.82, 200 x 200 x 64 (1.2) 3.86 / 3.71, 130 x 130 x 128 (1.2) 2.65 / 2.48; slabs of 256 x 256 x 32
 // (0.9, filter beside it) 30.8 / 28.7.
-static bool several_columns(const BpFastTables& t, const FastParams& P, int b_first, int b_count) {
+constexpr int kColumnRounds = 2;
+static bool several_columns(const BpFast& f, const BpFastGeom& g, int v, int b_first, int b_count) {
+  const FastVariant& fv = kFastVariants[v];
+  if (fv.seg != 2) return false;
+  if (f.cols[v] >= 0) return f.cols[v] != 0;
+  const BpFastTables& t = f.t[fv.table];
   long long blocks = 0;
   for (int b = b_first; b < b_first + b_count; ++b)
     if (t.h_zb.size() < 2 * (size_t)t.nblocks || t.h_zb[2 * b + 1] > 0) ++blocks;
-  const long long tiles = (long long)((P.XN + seg_tile_x(kSegCols) - 1) / seg_tile_x(kSegCols)) *
-                          ((P.YN + seg_tile_y(kSegCols) - 1) / seg_tile_y(kSegCols));
-  return tiles * blocks >= 2LL * kSegColsCtas * sm_count();
+  const long long tiles = (long long)((g.XN + seg_tile_x(kSegCols) - 1) / seg_tile_x(kSegCols)) *
+                          ((g.YN + seg_tile_y(kSegCols) - 1) / seg_tile_y(kSegCols));
+  return tiles * blocks >= (long long)kColumnRounds * seg_cols_per_sm(v) * sm_count();
+}
+
+void bp_fast_fix_columns(BpFast* f, const BpFastGeom& g) {
+  signed char cols[kFastVariants_n];
+  for (int v = 0; v < kFastVariants_n; ++v) {
+    f->cols[v] = -1;
+    cols[v] = several_columns(*f, g, v, 0, f->t[kFastVariants[v].table].nblocks);
+  }
+  std::copy(cols, cols + kFastVariants_n, f->cols);
 }
 
 // Launches variant v over z blocks [b_first, b_first + b_count) (count < 0: all).
@@ -1339,7 +1367,7 @@ static int run_variant(const BpFast& f, const BpFastGeom& g, int v, float* vol, 
     HR_REQUIRE(f.tex.kind == fv.tex && f.tex.views >= g.PN, "fast backprojection: the textures of variant %d are "
                "not prepared", v);
     if (fv.seg) {
-      const bool cols = fv.seg == 2 && several_columns(t, P, b_first, b_count);
+      const bool cols = several_columns(f, g, v, b_first, b_count);
       switch (v) {
         case 16: launch_tex_seg<8, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
         case 17: launch_tex_seg<4, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
@@ -1574,7 +1602,10 @@ static int pinned_variant() {
 }
 
 // Times every variant on the same middle band of 32 slices (all columns) and
-// keeps the fastest. The band is written into vol; synchronises the stream.
+// keeps the fastest; where a launch over the whole volume runs several columns
+// per thread, on a band of enough slices to run them too, so that the kernel
+// timed is the kernel kept. (A streamed execution's ranges may be smaller: they
+// go by their own size.) The band is written into vol; synchronises the stream.
 int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t* fpb, cudaStream_t s) {
   const int pin = pinned_variant();
   HR_REQUIRE(pin != -2, "HELIXRECON_BP_VARIANT must be an integer in [0, %d)", kFastVariants_n);
@@ -1594,8 +1625,14 @@ int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t*
   float fill_ms = 0.f;  // texture variants: filling the arrays, per slice of the volume
   for (int v = 0; v < kFastVariants_n && st == HR_OK; ++v) {
     const int nz = kFastNz[kFastVariants[v].table];
-    const int b0 = z_first / nz;
-    const int bc = std::min((band + nz - 1) / nz, f->t[kFastVariants[v].table].nblocks - b0);
+    const int nblocks = f->t[kFastVariants[v].table].nblocks;
+    int b0 = z_first / nz;
+    int bc = std::min((band + nz - 1) / nz, nblocks - b0);
+    f->tuned_cols[v] = several_columns(*f, g, v, 0, nblocks);
+    while (f->tuned_cols[v] && bc < nblocks && !several_columns(*f, g, v, b0, bc)) {
+      bc = std::min(bc + bc / 4 + 1, nblocks);
+      b0 = std::min(std::max(0, g.ZN / 2 / nz - bc / 2), nblocks - bc);
+    }
     if (kFastVariants[v].tex && f->tex.kind != kFastVariants[v].tex) {
       f->variant = v;
       st = bp_fast_tex_prepare(f, g);
@@ -1638,21 +1675,25 @@ int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t*
   return bp_fast_tex_prepare(f, g);
 }
 
-int bp_fast_describe(const BpFast& f, char* buf, int len) {
+int bp_fast_describe(const BpFast& f, const BpFastGeom& g, char* buf, int len) {
   if (!buf || len <= 0) return HR_OK;
   const FastVariant& fv = kFastVariants[f.variant];
+  // the form of a launch over the whole volume
+  const bool cols = several_columns(f, g, f.variant, 0, f.t[fv.table].nblocks);
   int n = snprintf(buf, (size_t)len, "slices_per_thread=%d gathers=%s tile=%dx%d %s", kFastNz[fv.table],
-                   fv.tex == kTexHalf ? (fv.seg == 2 ? (fv.occ ? "texture-fp16-segmented-four-columns-8ctas"
-                                                               : "texture-fp16-segmented-four-columns")
+                   fv.tex == kTexHalf ? (cols ? (fv.occ ? "texture-fp16-segmented-four-columns-8ctas"
+                                                        : "texture-fp16-segmented-four-columns")
+                                        : fv.seg == 2 ? (fv.occ ? "texture-fp16-segmented-two-views-6ctas"
+                                                                : "texture-fp16-segmented-two-views")
                                         : fv.seg ? (fv.occ ? "texture-fp16-segmented-6ctas" : "texture-fp16-segmented")
                                         : "texture-fp16")
                    : fv.tex == kTexFloat ? "texture-fp32"
                    : fv.chunk < 0 ? "paired-f32x2" : fv.chunk == 0 ? "per-slice" : fv.chunk == 4 ? "chunk4" : "chunk8",
-                   kBx, kBy, f.tuned == 2 ? "(pinned by HELIXRECON_BP_VARIANT)"
+                   cols ? seg_tile_x(kSegCols) : kBx, cols ? seg_tile_y(kSegCols) : kBy, f.tuned == 2 ? "(pinned by HELIXRECON_BP_VARIANT)"
                    : f.tuned ? "(autotuned; ms/slice:" : "(default)");
   if (f.tuned == 1) {
     for (int v = 0; v < kFastVariants_n && n > 0 && n < len; ++v)
-      n += snprintf(buf + n, (size_t)(len - n), " v%d=%.4f", v, f.tuned_ms[v]);
+      n += snprintf(buf + n, (size_t)(len - n), " v%d=%.4f%s", v, f.tuned_ms[v], f.tuned_cols[v] ? "x4" : "");
     if (n > 0 && n < len) snprintf(buf + n, (size_t)(len - n), ")");
   }
   return HR_OK;

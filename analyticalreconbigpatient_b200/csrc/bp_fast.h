@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -101,8 +102,13 @@ struct BpFast {
   int variant = kFastDefaultVariant;
   int tuned = 0;
   float tuned_ms[kFastVariants_n] = {};  // autotuner: ms per slice of each variant
+  bool tuned_cols[kFastVariants_n] = {};  // and whether it ran several columns per thread
+  // Whether launches of a variant run several columns per thread: -1 by the launch's size (bp_fast_fix_columns
+  // settles it, for launches captured once and replayed with other tables)
+  signed char cols[kFastVariants_n];
   size_t bytes = 0;
   BpFastTex tex;
+  BpFast() { std::fill(cols, cols + kFastVariants_n, (signed char)-1); }
 };
 
 struct BpFastHost {
@@ -123,7 +129,9 @@ int bp_fast_upload(BpFast* f, const BpFastHost& h, cudaStream_t s);
 void bp_fast_destroy(BpFast* f);
 int bp_fast_execute(const BpFast& f, const BpFastGeom& g, float* vol, const uint32_t* fpb, cudaStream_t s);
 int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t* fpb, cudaStream_t s);
-int bp_fast_describe(const BpFast& f, char* buf, int len);
+int bp_fast_describe(const BpFast& f, const BpFastGeom& g, char* buf, int len);
+// Settles the column form of every variant's launches from the tables as they are now.
+void bp_fast_fix_columns(BpFast* f, const BpFastGeom& g);
 // Allocates (or frees) the layered textures the plan's variant samples
 // (no-op for the gather variants); hr_bp_select and the slab pipeline call it
 // after choosing a variant by hand.

@@ -33,7 +33,6 @@
 // fan windows and writes only their slices; there is nothing to exchange.
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <vector>
 
 #include "bp_fast.h"
@@ -364,11 +363,14 @@ static int prepare(hr_slab_plan* p, const float* fan, int fan_view0, bool fan_on
   hr::BpFastHost h;
   HR_TRY(hr::bp_fast_host_tables(&h, slab_geom(p, k), p->w.data()));
   HR_TRY(hr::bp_fast_upload(&p->fast[b], h, p->sc));
+  hr::bp_fast_fix_columns(&p->fast[b], p->gslab);  // the graphs replay one form for every slab
   HR_TRY(slab_filter(p, b, p->sc));
   HR_TRY(hr::bp_fast_autotune(&p->fast[b], p->gslab, p->d_vslab[b], p->d_pairs[b], p->sc));
   p->fast[b ^ 1].variant = p->fast[b].variant;
   p->fast[b ^ 1].tuned = p->fast[b].tuned;
-  std::memcpy(p->fast[b ^ 1].tuned_ms, p->fast[b].tuned_ms, sizeof(p->fast[b].tuned_ms));
+  std::copy(p->fast[b].tuned_ms, p->fast[b].tuned_ms + hr::kFastVariants_n, p->fast[b ^ 1].tuned_ms);
+  std::copy(p->fast[b].tuned_cols, p->fast[b].tuned_cols + hr::kFastVariants_n, p->fast[b ^ 1].tuned_cols);
+  std::copy(p->fast[b].cols, p->fast[b].cols + hr::kFastVariants_n, p->fast[b ^ 1].cols);
   HR_TRY(hr::bp_fast_tex_prepare(&p->fast[b ^ 1], p->gslab));
   HR_CUDA_TRY(cudaStreamSynchronize(p->sc));
   HR_CUDA_TRY(cudaStreamSynchronize(p->scopy));
@@ -449,7 +451,7 @@ extern "C" int hr_slab_fan_range(const hr_slab_plan* p, int* first_view, int* nv
 extern "C" int hr_slab_describe(const hr_slab_plan* p, char* buf, int len) {
   HR_REQUIRE(p != nullptr, "hr_slab_describe: NULL plan");
   char bp[640];
-  HR_TRY(hr::bp_fast_describe(p->fast[0], bp, sizeof(bp)));
+  HR_TRY(hr::bp_fast_describe(p->fast[0], p->gslab, bp, sizeof(bp)));
   if (buf && len > 0) {
     char part[96] = "";
     if (p->nparts > 1)
