@@ -1319,39 +1319,48 @@ static int seg_cols_per_sm(K kern) {
   return std::max(n, 1);
 }
 static int seg_cols_per_sm(int v) {
-  static const int n18 = seg_cols_per_sm(bp_tex_seg_kernel<8, kSegCols, 1>);
   static const int n19 = seg_cols_per_sm(bp_tex_seg_kernel<4, kSegCols, 1>);
   static const int n21 = seg_cols_per_sm(bp_tex_seg_occ_kernel<4, kSegCols, 1>);
-  return v == 18 ? n18 : v == 19 ? n19 : n21;
+  return v == 19 ? n19 : n21;
 }
 
-// Whether a launch over z blocks [b_first, b_first + b_count) has the CTAs for kSegCols columns per thread: two
-// rounds of them, blocks without views not counted. Fewer leave SMs idle at the end, and beside another kernel (a
-// slab's or chunk's filter) one round of long CTAs keeps that kernel out until it ends. Measured, several columns
-// against two views: 512 x 512 x 16 (1.7 rounds) 4.80 / 5.00 ms, 301 x 301 x 40 (1.6) 4.64 / 4.71, 256 x 256 x 24
-// (0.6) 1.82 / 1.82, 200 x 200 x 64 (1.2) 3.86 / 3.71, 130 x 130 x 128 (1.2) 2.65 / 2.48; slabs of 256 x 256 x 32
-// (0.9, filter beside it) 30.8 / 28.7.
-constexpr int kColumnRounds = 2;
-static bool several_columns(const BpFast& f, const BpFastGeom& g, int v, int b_first, int b_count) {
-  const FastVariant& fv = kFastVariants[v];
-  if (fv.seg != 2) return false;
-  if (f.cols[v] >= 0) return f.cols[v] != 0;
-  const BpFastTables& t = f.t[fv.table];
+// Whether a launch of variant v over z blocks [b_first, b_first + b_count) runs kSegCols columns per thread.
+//
+// By its size: from two rounds of CTAs on (blocks without views not counted). Measured, variant 21, four columns
+// against two views, ms a call: alone the line would be 1.5 rounds (512 x 512: 1.3 rounds 2.38 / 2.47, 1.7 2.98 /
+// 3.19, 3.9 6.28 / 6.78; 301 x 301: 1.1 2.38 / 2.17, 1.3 2.43 / 2.41, 1.6 2.82 / 2.93, 4.0 6.41 / 6.79), but beside
+// another kernel (a slab's filter), which a round of long CTAs keeps out until it ends, it is two: slabs of 256 x 256
+// x 56 at 3.92 mm (1.5 rounds) 15.7 / 14.5, x 64 (1.7) 16.0 / 15.6, 301 x 301 x 40 (1.6) 23.2 / 22.6, x 48 (1.9) 21.7 /
+// 21.7, 512 x 512 x 16 (1.7) 27.2 / 27.9.
+//
+// By the grid and the slices: small grids, rows that end inside a thread's columns and thick slices cost more than
+// that line tells (2 to 4 rounds: 200 x 200 3.47 / 3.41 to 6.31 / 6.44, 230 x 230 at 2 mm 3.99 / 3.82 to 7.13 / 7.05,
+// 165 x 165 at 2 mm 4.52 / 4.04 to 7.49 / 6.77, 130 x 130 3.61 / 3.34 to 6.45 / 6.24). So the autotuner times both
+// forms; an untuned plan takes four columns where they leave at most 2.5 % more lanes idle.
+//
+// (Eight slices and four columns, 18's table, need registers for 5 CTAs: 512 x 512 at 3.92 mm, 3.9 rounds, 7.78 / 7.59,
+// thin slices 6.41 / 6.69 where 21 takes 6.28.)
+static bool columns_by_size(const BpFast& f, const BpFastGeom& g, int v, int b_first, int b_count, int rounds) {
+  const BpFastTables& t = f.t[kFastVariants[v].table];
   long long blocks = 0;
   for (int b = b_first; b < b_first + b_count; ++b)
     if (t.h_zb.size() < 2 * (size_t)t.nblocks || t.h_zb[2 * b + 1] > 0) ++blocks;
   const long long tiles = (long long)((g.XN + seg_tile_x(kSegCols) - 1) / seg_tile_x(kSegCols)) *
                           ((g.YN + seg_tile_y(kSegCols) - 1) / seg_tile_y(kSegCols));
-  return tiles * blocks >= (long long)kColumnRounds * seg_cols_per_sm(v) * sm_count();
+  return tiles * blocks >= (long long)rounds * seg_cols_per_sm(v) * sm_count();
+}
+constexpr int kColumnRounds = 2;
+static bool several_columns(const BpFast& f, const BpFastGeom& g, int v, int b_first, int b_count) {
+  if (kFastVariants[v].seg != 3 || f.cols[v] == kColsNever) return false;
+  if (f.cols[v] == kColsAlways) return true;
+  const long long wide = (g.YN + 4 * kSegCols - 1) / (4 * kSegCols) * kSegCols, thin = (g.YN + 3) / 4;  // warps' rows
+  if (f.cols[v] == kColsRule && wide * 40 > thin * 41) return false;
+  return columns_by_size(f, g, v, b_first, b_count, kColumnRounds);
 }
 
 void bp_fast_fix_columns(BpFast* f, const BpFastGeom& g) {
-  signed char cols[kFastVariants_n];
-  for (int v = 0; v < kFastVariants_n; ++v) {
-    f->cols[v] = -1;
-    cols[v] = several_columns(*f, g, v, 0, f->t[kFastVariants[v].table].nblocks);
-  }
-  std::copy(cols, cols + kFastVariants_n, f->cols);
+  for (int v = 0; v < kFastVariants_n; ++v)
+    f->cols[v] = several_columns(*f, g, v, 0, f->t[kFastVariants[v].table].nblocks) ? kColsAlways : kColsNever;
 }
 
 // Launches variant v over z blocks [b_first, b_first + b_count) (count < 0: all).
@@ -1371,10 +1380,7 @@ static int run_variant(const BpFast& f, const BpFastGeom& g, int v, float* vol, 
       switch (v) {
         case 16: launch_tex_seg<8, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
         case 17: launch_tex_seg<4, 1, 1, false>(t, f, P, vol, b_first, b_count, s); break;
-        case 18:
-          cols ? launch_tex_seg<8, kSegCols, 1, false>(t, f, P, vol, b_first, b_count, s)
-               : launch_tex_seg<8, 1, 2, false>(t, f, P, vol, b_first, b_count, s);
-          break;
+        case 18: launch_tex_seg<8, 1, 2, false>(t, f, P, vol, b_first, b_count, s); break;
         case 19:
           cols ? launch_tex_seg<4, kSegCols, 1, false>(t, f, P, vol, b_first, b_count, s)
                : launch_tex_seg<4, 1, 2, false>(t, f, P, vol, b_first, b_count, s);
@@ -1602,11 +1608,17 @@ static int pinned_variant() {
 }
 
 // Times every variant on the same middle band of 32 slices (all columns) and
-// keeps the fastest; where a launch over the whole volume runs several columns
-// per thread, on a band of enough slices to run them too, so that the kernel
-// timed is the kernel kept. (A streamed execution's ranges may be smaller: they
-// go by their own size.) The band is written into vol; synchronises the stream.
+// keeps the fastest. A variant that may run several columns per thread is timed
+// both ways and keeps the faster form, on a band of two rounds of CTAs: the
+// kernel timed is the kernel kept. (A streamed execution's ranges, and slabs'
+// partial ones, may be smaller: the former go by their own size.) The texture
+// variants come first, each copy's together, so that a copy is made once and the
+// others, usually slower, end after one repeat. The band is written into vol;
+// synchronises the stream.
+constexpr int kTuneOrder[] = {14, 15, 11, 12, 13, 16, 17, 18, 19, 20, 21, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10};
+static_assert(sizeof(kTuneOrder) / sizeof(kTuneOrder[0]) == kFastVariants_n, "every variant once");
 int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t* fpb, cudaStream_t s) {
+  std::fill(f->cols, f->cols + kFastVariants_n, kColsRule);
   const int pin = pinned_variant();
   HR_REQUIRE(pin != -2, "HELIXRECON_BP_VARIANT must be an integer in [0, %d)", kFastVariants_n);
   if (pin >= 0) {
@@ -1623,13 +1635,15 @@ int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t*
   int best_v = f->variant;
   int st = HR_OK;
   float fill_ms = 0.f;  // texture variants: filling the arrays, per slice of the volume
-  for (int v = 0; v < kFastVariants_n && st == HR_OK; ++v) {
+  for (const int v : kTuneOrder) {
+    if (st != HR_OK) break;
     const int nz = kFastNz[kFastVariants[v].table];
     const int nblocks = f->t[kFastVariants[v].table].nblocks;
     int b0 = z_first / nz;
     int bc = std::min((band + nz - 1) / nz, nblocks - b0);
-    f->tuned_cols[v] = several_columns(*f, g, v, 0, nblocks);
-    while (f->tuned_cols[v] && bc < nblocks && !several_columns(*f, g, v, b0, bc)) {
+    // forms to time: the variant's only one, or two views and several columns
+    const bool both = kFastVariants[v].seg == 3 && columns_by_size(*f, g, v, 0, nblocks, kColumnRounds);
+    while (both && bc < nblocks && !columns_by_size(*f, g, v, b0, bc, kColumnRounds)) {
       bc = std::min(bc + bc / 4 + 1, nblocks);
       b0 = std::min(std::max(0, g.ZN / 2 / nz - bc / 2), nblocks - bc);
     }
@@ -1647,16 +1661,24 @@ int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t*
         fill_ms = t / (float)std::max(g.ZN_valid, 1);
       }
     }
-    float ms = 1e30f;
-    for (int rep = 0; rep < 3 && st == HR_OK; ++rep) {
-      cudaEventRecord(e0, s);
-      st = run_variant(*f, g, v, vol, fpb, b0, bc, s);
-      cudaEventRecord(e1, s);
-      if (cudaEventSynchronize(e1) != cudaSuccess) st = hr::fail(HR_ERR_CUDA, "fast backprojection autotune failed");
-      float t = 0.f;
-      cudaEventElapsedTime(&t, e0, e1);
-      if (rep > 0) ms = std::min(ms, t / (float)(bc * nz) + (kFastVariants[v].tex ? fill_ms : 0.f));  // per slice
+    float form_ms[2] = {1e30f, 1e30f};
+    for (int form = 0; form <= (both ? 1 : 0) && st == HR_OK; ++form) {
+      f->cols[v] = form == 0 ? kColsNever : kColsAlways;
+      float& ms = form_ms[form];
+      for (int rep = 0; rep < (both ? 2 : 3) && st == HR_OK; ++rep) {
+        cudaEventRecord(e0, s);
+        st = run_variant(*f, g, v, vol, fpb, b0, bc, s);
+        cudaEventRecord(e1, s);
+        if (cudaEventSynchronize(e1) != cudaSuccess) st = hr::fail(HR_ERR_CUDA, "fast backprojection autotune failed");
+        float t = 0.f;
+        cudaEventElapsedTime(&t, e0, e1);
+        if (rep > 0) ms = std::min(ms, t / (float)(bc * nz) + (kFastVariants[v].tex ? fill_ms : 0.f));  // per slice
+        if (rep > 0 && ms > 1.5f * best) break;  // no repeat brings it back
+      }
     }
+    f->tuned_cols[v] = both && form_ms[1] < form_ms[0];
+    const float ms = std::min(form_ms[0], form_ms[1]);
+    f->cols[v] = f->tuned_cols[v] ? kColsTuned : both ? kColsNever : kColsRule;
     f->tuned_ms[v] = ms;
     if (ms < best) {
       best = ms;
@@ -1668,6 +1690,7 @@ int bp_fast_autotune(BpFast* f, const BpFastGeom& g, float* vol, const uint32_t*
   f->variant = best_v;
   if (st != HR_OK) {
     f->variant = kFastDefaultVariant;
+    std::fill(f->cols, f->cols + kFastVariants_n, kColsRule);
     tex_free(&f->tex);
     return st;
   }
@@ -1683,7 +1706,7 @@ int bp_fast_describe(const BpFast& f, const BpFastGeom& g, char* buf, int len) {
   int n = snprintf(buf, (size_t)len, "slices_per_thread=%d gathers=%s tile=%dx%d %s", kFastNz[fv.table],
                    fv.tex == kTexHalf ? (cols ? (fv.occ ? "texture-fp16-segmented-four-columns-8ctas"
                                                         : "texture-fp16-segmented-four-columns")
-                                        : fv.seg == 2 ? (fv.occ ? "texture-fp16-segmented-two-views-6ctas"
+                                        : fv.seg >= 2 ? (fv.occ ? "texture-fp16-segmented-two-views-6ctas"
                                                                 : "texture-fp16-segmented-two-views")
                                         : fv.seg ? (fv.occ ? "texture-fp16-segmented-6ctas" : "texture-fp16-segmented")
                                         : "texture-fp16")

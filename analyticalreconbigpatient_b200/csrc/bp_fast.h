@@ -36,11 +36,11 @@ constexpr int kTexHalf = 1, kTexFloat = 2;
 // a z block runs in segments over which the set of slices whose window holds
 // the view is a fixed range [ma, mb], with code specialised for that range, so
 // slices without the view cost nothing (thick slices: a block's union window
-// is much longer than one slice's); seg = 2: the same with four columns per
-// thread, which share what a view costs apart from its taps, or, in launches
-// too small for that, with two views per iteration in segments of at most four
-// slices. occ: registers bounded for 6 CTAs per SM (8 of half the threads with
-// four columns).
+// is much longer than one slice's); seg = 2: the same with two views per
+// iteration in segments of at most four slices; seg = 3: with four columns per
+// thread, which share what a view costs apart from its taps, or, in launches too
+// small for that, as 2. occ: registers bounded for 6 CTAs per SM (8 of half the
+// threads with four columns).
 struct FastVariant {
   int table, chunk, tex, seg, occ;
 };
@@ -49,8 +49,8 @@ constexpr FastVariant kFastVariants[] = {{0, 0}, {0, 4}, {0, 8}, {1, 0}, {1, 4},
                                          {1, 0, kTexHalf}, {0, 0, kTexHalf}, {2, 0, kTexHalf},
                                          {1, 0, kTexFloat}, {0, 0, kTexFloat},
                                          {1, 0, kTexHalf, 1}, {2, 0, kTexHalf, 1},
-                                         {1, 0, kTexHalf, 2}, {2, 0, kTexHalf, 2},
-                                         {1, 0, kTexHalf, 1, 6}, {2, 0, kTexHalf, 2, 8}};
+                                         {1, 0, kTexHalf, 2}, {2, 0, kTexHalf, 3},
+                                         {1, 0, kTexHalf, 1, 6}, {2, 0, kTexHalf, 3, 8}};
 constexpr int kFastVariants_n = sizeof(kFastVariants) / sizeof(kFastVariants[0]);
 constexpr int kFastDefaultVariant = 0;
 
@@ -95,6 +95,10 @@ struct BpFastTex {
   size_t bytes = 0;
 };
 
+// Several columns per thread: by the launch's size and the grid (untuned plans), never, always (launches captured
+// once and replayed with other tables), or by the size alone (timed, and faster).
+constexpr signed char kColsRule = -1, kColsNever = 0, kColsAlways = 1, kColsTuned = 2;
+
 struct BpFast {
   BpFastTables t[kFastTableSets];
   float2* d_trig = nullptr;  // per view: {cos, sin}
@@ -103,12 +107,11 @@ struct BpFast {
   int tuned = 0;
   float tuned_ms[kFastVariants_n] = {};  // autotuner: ms per slice of each variant
   bool tuned_cols[kFastVariants_n] = {};  // and whether it ran several columns per thread
-  // Whether launches of a variant run several columns per thread: -1 by the launch's size (bp_fast_fix_columns
-  // settles it, for launches captured once and replayed with other tables)
+  // Which launches of a variant run several columns per thread (kCols...)
   signed char cols[kFastVariants_n];
   size_t bytes = 0;
   BpFastTex tex;
-  BpFast() { std::fill(cols, cols + kFastVariants_n, (signed char)-1); }
+  BpFast() { std::fill(cols, cols + kFastVariants_n, kColsRule); }
 };
 
 struct BpFastHost {

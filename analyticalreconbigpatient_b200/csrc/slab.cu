@@ -363,9 +363,9 @@ static int prepare(hr_slab_plan* p, const float* fan, int fan_view0, bool fan_on
   hr::BpFastHost h;
   HR_TRY(hr::bp_fast_host_tables(&h, slab_geom(p, k), p->w.data()));
   HR_TRY(hr::bp_fast_upload(&p->fast[b], h, p->sc));
-  hr::bp_fast_fix_columns(&p->fast[b], p->gslab);  // the graphs replay one form for every slab
   HR_TRY(slab_filter(p, b, p->sc));
   HR_TRY(hr::bp_fast_autotune(&p->fast[b], p->gslab, p->d_vslab[b], p->d_pairs[b], p->sc));
+  hr::bp_fast_fix_columns(&p->fast[b], p->gslab);  // the graphs replay one form for every slab
   p->fast[b ^ 1].variant = p->fast[b].variant;
   p->fast[b ^ 1].tuned = p->fast[b].tuned;
   std::copy(p->fast[b].tuned_ms, p->fast[b].tuned_ms + hr::kFastVariants_n, p->fast[b ^ 1].tuned_ms);

@@ -216,10 +216,10 @@ int hr_bp_describe(const hr_bp_plan* plan, char* buf, int len);
  * eight / sixteen with an FP32 copy, 16-17 eight / four slices per thread
  * from the FP16 copy with the view loop cut into segments of a fixed set of
  * slices holding the view (thick slices), 18-19 eight / four slices per
- * thread as 16-17 with four columns per thread (which share the work of a
- * view apart from its taps) or, in launches too small for that, two views per
- * iteration in segments of at most four slices, 20 as 16 and 21 as 19 with
- * registers bounded for more CTAs per SM; the texture variants allocate the
+ * thread as 16-17 with two views per iteration in segments of at most four
+ * slices or, 19 in launches large enough for it, with four columns per thread
+ * (which share the work of a view apart from its taps), 20 as 16 and 21 as 19
+ * with registers bounded for more CTAs per SM; the texture variants allocate the
  * copy, 2 or 4 bytes per sample, and fill it on every execution).
  * For tests and manual tuning. */
 int hr_bp_select(hr_bp_plan* plan, int variant);

@@ -1,5 +1,6 @@
-"""Which form of the segmented texture kernels a plan times and runs: the autotuner times a variant in the form (four
-columns per thread, or two views per iteration) that a launch over the plan's volume runs, and describe() names it."""
+"""Which form of the segmented texture kernels a plan times and runs: the autotuner's time of a variant is that of the
+form (four columns per thread, or two views per iteration) that a launch over the plan's volume runs, and describe()
+names it; four columns only where the launch has the CTAs, and, untuned, where the grid fills their threads."""
 import ctypes
 import re
 
@@ -39,7 +40,21 @@ def test_the_form_timed_is_the_form_run(cuda, N, ZN, four):
     forms = _forms(plans, (18, 19, 21))
     plans.close()
     assert all(t == r for t, r in forms.values()), forms
-    assert forms[21][1] == four, forms
+    assert not forms[18][1] and (four or not any(r for _, r in forms.values())), forms
+
+
+@pytest.mark.parametrize("N,ZN,four", [(512, 40, True), (509, 40, True), (256, 80, True), (256, 36, False),
+                                       (130, 400, False), (165, 300, False)])
+def test_the_form_of_an_untuned_plan(cuda, N, ZN, four):
+    """130 and 165 rows of pixels leave 9 and 5 % of the lanes of four-column threads idle."""
+    sc = G.Scan(ZL=8, N_2pi=246, pitch=0.9375, rotations=26, XN=N, YN=N, ZN=ZN, dx=500.0 / N, dy=500.0 / N, dz=0.25)
+    plans = StagePlans(sc, _lib.HR_FORM_FAST)
+    buf = ctypes.create_string_buffer(1024)
+    for v in (18, 19, 21):
+        _lib.check(_lib.load().hr_bp_select(plans._bp, v))
+        _lib.check(_lib.load().hr_bp_describe(plans._bp, buf, 1024))
+        assert ("four-columns" in buf.value.decode()) == (four and v != 18), (v, buf.value)
+    plans.close()
 
 
 @pytest.mark.parametrize("slab,four", [(80, True), (24, False)])
