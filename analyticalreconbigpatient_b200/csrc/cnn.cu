@@ -545,7 +545,7 @@ constexpr int kWgThreads = 32 * (kWgWorkers + 2);
 constexpr int kWgTmemCols = 512;
 constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256;
 
-template <int CIN, int COUT, bool RAGGED>
+template <int CIN, int COUT>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __restrict__ X,
                                                                  const uint4* __restrict__ Gr,
                                                                  const uint4* __restrict__ zero, int B, int H, int W,
@@ -564,9 +564,18 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int Wp = padded_width(W);
+  const uint32_t nseg = (uint32_t)(W + kTileM - 1) / kTileM, npair = (uint32_t)(H + 1) / 2;
+  // pixels of this CTA's tiles: where a row's last strip is short, all of a CTA's tiles are the same strip
+  const int np = W % kTileM == 0 ? kTileM : min(W - (int)(blockIdx.x % nseg) * kTileM, kTileM);
   if constexpr (XC * 4 < kWgXPlanes) {  // planes no copy fills are read as rows of D that nobody uses
     for (int i = tid; i < kWgStages * kWgStage / 16; i += kWgThreads)
       reinterpret_cast<uint4*>(wg_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  } else if (np < kTileM) {  // and pixels no copy fills stay zeros in both operands
+    for (int i = warp; i < kWgStages * (kWgXPlanes + kWgGPlanes); i += kWgThreads / 32)
+      for (int k = np + lane; k < kTileM + 2; k += 32)
+        reinterpret_cast<uint4*>(wg_smem + (size_t)i * kWgPlane)[k] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (tid == 0) {
@@ -594,15 +603,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
   const uint32_t tmem = *tmem_slot;
   const uint32_t smem0 = smem_u32(wg_smem);
 
-  const int Wp = padded_width(W);
-  const uint32_t nseg = (uint32_t)(W + kTileM - 1) / kTileM, npair = (uint32_t)(H + 1) / 2;
   const uint32_t tiles = (uint32_t)B * npair * nseg;                                 // < 2^31, checked at launch
   const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);             // this CTA's (grid <= tiles)
-  // pixels of this CTA's i-th tile: with ragged widths a row's last strip is short, and the sums stop with it
-  auto tile_pixels = [&](int i) {
-    if constexpr (!RAGGED) return kTileM;
-    return min(W - (int)((blockIdx.x + (uint32_t)i * gridDim.x) % nseg) * kTileM, kTileM);
-  };
 
   if (warp < kWgWorkers) {
     // ---- bias sums and flushes -------------------------------------------------------------------
@@ -642,7 +644,6 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
     const int gc = tid % GC, gp = tid / GC;
     for (int j = 0; j < n && ok; ++j) {
       const int s = j % kWgStages;
-      const int np = tile_pixels(j);
       const bool waited =
           lane != 0 || mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
       if (!__all_sync(0xffffffffu, waited)) {
@@ -654,8 +655,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       for (int row = 0; row < 2; ++row)
 #pragma unroll
         for (int px = 0; px < kTileM; px += 32 * kWgWorkers / GC) {
-          uint4 w = *reinterpret_cast<const uint4*>(st + (row * GC + gc) * kWgPlane + (gp + px) * 16);
-          if (RAGGED && gp + px >= np) w = make_uint4(0u, 0u, 0u, 0u);
+          const uint4 w = *reinterpret_cast<const uint4*>(st + (row * GC + gc) * kWgPlane + (gp + px) * 16);
           const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -695,7 +695,6 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       for (int j = 0; j < n && ok; ++j) {
         const int s = j % kWgStages, grp = j / kWgGroup, b = grp & 1;
         const bool first = j % kWgGroup == 0;
-        const int np = tile_pixels(j);
         if (first && grp >= 2)
           ok = mbar_wait(&tempty[b], (uint32_t)((grp >> 1) - 1) & 1, abort_flag, err, kWaitLimit);
         if (ok) ok = mbar_wait(&full[s], (uint32_t)(j / kWgStages) & 1, abort_flag, err, kWaitLimit);
@@ -706,18 +705,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
         // an offset of 16 bytes is one unit of a descriptor's address
         const uint64_t ad = desc_noswz(xa, 128, kWgPlane), bd = desc_noswz(ga, 128, kWgPlane);
         const uint32_t acc = tmem + b * 3 * kN;
-        if (!RAGGED || np == kTileM) {
 #pragma unroll
-          for (int ks = 0; ks < kTileM / 16; ++ks)
+        for (int ks = 0; ks < kTileM / 16; ++ks)
 #pragma unroll
-            for (int dx = 0; dx < 3; ++dx)
-              umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
-        } else {
-          for (int ks = 0; ks < (np + 15) / 16; ++ks)
-#pragma unroll
-            for (int dx = 0; dx < 3; ++dx)
-              umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
-        }
+          for (int dx = 0; dx < 3; ++dx)
+            umma(acc + dx * kN, ad + (ks * 16 + dx), bd + ks * 16, kIdesc, first && ks == 0 ? 0u : 1u);
         umma_commit(&empty[s]);
         if (j % kWgGroup == kWgGroup - 1 || j == n - 1) umma_commit(&tfull[b]);
       }
@@ -739,17 +731,6 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       if (!__all_sync(0xffffffffu, free)) break;
       const uint32_t t = blockIdx.x + (uint32_t)i * gridDim.x, by = t / nseg;
       const int x0 = (int)(t - by * nseg) * kTileM, b = (int)(by / npair), y = 2 * (int)(by - (uint32_t)b * npair);
-      const int np = RAGGED ? min(W - x0, kTileM) : kTileM;
-      const uint32_t d = dst + (uint32_t)s * kWgStage;
-      if (RAGGED && np % 16 != 0) {  // zeros, in both operands, for the pixels that the last MMA of a short strip has too many
-        if (lane < 4 * XC + 2 * GC)
-          for (int k = np; k < ((np + 15) & ~15); ++k)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(d + (uint32_t)(xrow ? k + 2 : k) * 16),
-                         "r"(0)
-                         : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-      }
       if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(4 * XC * (np + 2) + 2 * GC * np) * 16);
       __syncwarp();
       if (lane < 4 * XC + 2 * GC) {
@@ -757,7 +738,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
         const uint4* src = zero;
         if (yy >= 0 && yy < H)
           src = xrow ? X + plane_row(b, H, yy, XC, c, Wp) + x0 : Gr + plane_row(b, H, yy, GC, c, Wp) + x0 + 1;
-        bulk_load(d, src, (uint32_t)(xrow ? np + 2 : np) * 16, &full[s]);
+        bulk_load(dst + (uint32_t)s * kWgStage, src, (uint32_t)(xrow ? np + 2 : np) * 16, &full[s]);
       }
       issued = i + 1;
     }
@@ -971,24 +952,19 @@ int launch_conv(ConvArgs& a, cudaStream_t s) {
   return launch_dependent(conv_tc_kernel<CIN, COUT, EPI>, (unsigned)grid, kThreads, smem, s, a);
 }
 
-template <int CIN, int COUT, bool RAGGED>
-int launch_wgrad_of(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
-                    int* err, cudaStream_t s) {
-  const long long tiles = (long long)B * ((H + 1) / 2) * ((W + kTileM - 1) / kTileM);
-  const long long grid = std::min<long long>(tiles, hr::sm_count());
-  if (grid <= 0) return HR_OK;
-  HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
-  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT, RAGGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kWgSmem));
-  return launch_dependent(wgrad_tc_kernel<CIN, COUT, RAGGED>, (unsigned)grid, kWgThreads, kWgSmem, s, X, Gr, zero, B,
-                          H, W, dW, db, err);
-}
-
 template <int CIN, int COUT>
 int launch_wgrad(const uint4* X, const uint4* Gr, const uint4* zero, int B, int H, int W, float* dW, float* db,
                  int* err, cudaStream_t s) {
-  if (W % kTileM) return launch_wgrad_of<CIN, COUT, true>(X, Gr, zero, B, H, W, dW, db, err, s);
-  return launch_wgrad_of<CIN, COUT, false>(X, Gr, zero, B, H, W, dW, db, err, s);
+  const long long tiles = (long long)B * ((H + 1) / 2) * ((W + kTileM - 1) / kTileM);
+  long long grid = std::min<long long>(tiles, hr::sm_count());
+  if (grid <= 0) return HR_OK;
+  const long long nseg = (W + kTileM - 1) / kTileM;
+  if (W % kTileM) grid = std::max(grid / nseg, 1LL) * nseg;  // every CTA keeps one strip (tiles is such a multiple too)
+  HR_REQUIRE(tiles < (1LL << 31), "conv weight gradients: %lld tiles exceed one launch", tiles);
+  HR_CUDA_TRY(cudaFuncSetAttribute(wgrad_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kWgSmem));
+  return launch_dependent(wgrad_tc_kernel<CIN, COUT>, (unsigned)grid, kWgThreads, kWgSmem, s, X, Gr, zero, B, H, W,
+                          dW, db, err);
 }
 
 }  // namespace
