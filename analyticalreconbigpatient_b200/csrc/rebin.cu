@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) rebin_kernel(float* __restrict__ out, con
 // 1-2 ulp away from the reference on a quarter of the samples: they do not
 // round like the scalar mul.rn / add.rn sequence.)
 //
-// A thread walks `chunk` consecutive output views of its channel. The upper fan
+// A thread walks `chunk` (4 or 1) consecutive output views of its channel. The upper fan
 // view of one is the lower fan view of the next (the two angle steps are equal,
 // or nearly: where rounding, or DeltaTheta != DeltaFai, makes it another one,
 // the test on XB sees it), so its two channels' rows stay in registers and each
@@ -131,8 +131,13 @@ __global__ void __launch_bounds__(256) rebin_kernel(float* __restrict__ out, con
 // 188.8 -> 162.4 us with chunk = 4 (5.5 TB/s of compulsory traffic, 0.84 of a
 // plain copy's); 888 x 16, four: 107 -> 85.7. Chunks of 2, 8, 16: 164.8, 169.2,
 // 172.8 and 90.6, 87.0, 94.8 us: shorter ones read more rows, longer ones leave
-// fewer loads in flight.
+// fewer loads in flight. In launches that latency bounds, of fewer than some six
+// CTAs per SM with a view each (eight are one round), the walk only makes it
+// longer, and chunk is 1: 888 x 16, 4 views 2.06 us against 3.49 with 4 views per
+// thread, 64 views (3 CTAs per SM) 3.37 / 3.94, 100 (4.7) 4.6 / 5.3, 150 (7.1) 6.0 /
+// 5.3, 250 (11.8) 8.5 / 7.0; 300 x 32, 150 views (5.1) 4.2 / 4.8, 200 (6.8) 5.0 / 4.8.
 constexpr int kViewChunk = 4;
+constexpr int kWalkCtas = 6;  // per SM
 
 template <int NQ>
 __global__ void __launch_bounds__(256) rebin_rows_kernel(float* __restrict__ out, const float* __restrict__ proj,
@@ -278,7 +283,7 @@ int hr::rebin_execute_range(const hr_rebin_plan* p, float* d_out, const float* d
   const int nkq = nq ? p->ZL / (4 * nq) : p->ZL;
   const int threads = 256;
   const int gx = (p->YL * nkq + threads - 1) / threads;
-  const int chunk = nq ? kViewChunk : 1;
+  const int chunk = nq && (long long)gx * (i1 - i0) > (long long)kWalkCtas * hr::sm_count() ? kViewChunk : 1;
   int gy = std::min((i1 - i0 + chunk - 1) / chunk, 65535);  // the kernels stride over the views
   if (max_ctas > 0) gy = std::max(1, std::min(gy, max_ctas / gx));
   const dim3 grid(gx, gy);
