@@ -825,6 +825,7 @@ size_t plain_q_smem(const BpParams& P) {
 // plan: every launch sets it to this most, so that of two plans executed by two
 // threads neither lowers it between the other's setting and launch.
 constexpr size_t kPlainQSmemMax = 96 * 1024;
+bool plain_q_fits(const BpParams& P) { return P.qcap > 0 && plain_q_smem(P) <= kPlainQSmemMax; }
 
 // Dynamic shared memory of bp_fp64_q_kernel, and the most it may take (two CTAs per SM still fit); above
 // it (thick slices) the per-update kernel runs.
@@ -834,6 +835,7 @@ size_t fp64_q_smem(const BpParams& P) {
          sizeof(double) * (size_t)P.qcap * kNzFp64Q;
 }
 constexpr size_t kFp64QSmemMax = 100 * 1024;
+bool fp64_q_fits(const BpParams& P) { return P.qcap > 0 && fp64_q_smem(P) <= kFp64QSmemMax; }
 
 // The plain-form launch of both the plan and the allocation-free entry (the
 // same kernel for the same geometry, so their results are identical).
@@ -841,13 +843,12 @@ int launch_plain(const BpParams& P, float* vol, const float* fp, const ViewTab* 
                  cudaStream_t s) {
   dim3 grid((P.XN + kBx - 1) / kBx, (P.YN + kBy - 1) / kBy, (P.ZN + kNzPlain - 1) / kNzPlain);
   HR_REQUIRE(grid.z <= 65535 && grid.y <= 65535, "backprojection: grid too large");
-  const size_t qsmem = plain_q_smem(P);
-  if (P.qcap > 0 && qsmem <= kPlainQSmemMax) {
+  if (plain_q_fits(P)) {
     grid.x = (P.XN + kTx - 1) / kTx;
     grid.y = (P.YN + kTy - 1) / kTy;
     HR_CUDA_TRY(cudaFuncSetAttribute(bp_plain_q_kernel<kNzPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kPlainQSmemMax));
-    bp_plain_q_kernel<kNzPlain><<<grid, dim3(kTx, kTy), qsmem, s>>>(vol, fp, views, w, P);
+    bp_plain_q_kernel<kNzPlain><<<grid, dim3(kTx, kTy), plain_q_smem(P), s>>>(vol, fp, views, w, P);
   } else {
     bp_plain_kernel<kNzPlain><<<grid, dim3(kBx, kBy), sizeof(float) * P.N_2pi, s>>>(vol, fp, views, w, P);
   }
@@ -940,12 +941,11 @@ extern "C" int hr_bp_execute(const hr_bp_plan* pl, void* d_vol, const void* d_fp
     HR_REQUIRE(grid.z <= 65535 && grid.y <= 65535, "backprojection: grid too large");
     double* vol = static_cast<double*>(d_vol);
     const double* fp = static_cast<const double*>(d_fp);
-    const size_t qsmem = fp64_q_smem(P);
-    if (P.qcap > 0 && qsmem <= kFp64QSmemMax) {
+    if (fp64_q_fits(P)) {
       grid = dim3((P.XN + kDx - 1) / kDx, (P.YN + kDy - 1) / kDy, (P.ZN + kNzFp64Q - 1) / kNzFp64Q);
       HR_CUDA_TRY(cudaFuncSetAttribute(bp_fp64_q_kernel<kNzFp64Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kFp64QSmemMax));
-      bp_fp64_q_kernel<kNzFp64Q><<<grid, dim3(kDx, kDy), qsmem, s>>>(vol, fp, pl->d_views, pl->d_wd, P);
+      bp_fp64_q_kernel<kNzFp64Q><<<grid, dim3(kDx, kDy), fp64_q_smem(P), s>>>(vol, fp, pl->d_views, pl->d_wd, P);
     } else {
       bp_fp64_kernel<kNzFp64><<<grid, dim3(kBx, kBy), sizeof(double) * P.N_2pi, s>>>(vol, fp, pl->d_views, pl->d_wd,
                                                                                     P);
@@ -982,12 +982,12 @@ extern "C" int hr_bp_select(hr_bp_plan* pl, int variant) {
 extern "C" int hr_bp_describe(const hr_bp_plan* pl, char* buf, int len) {
   HR_REQUIRE(pl != nullptr, "hr_bp_describe: NULL plan");
   if (pl->form == HR_FORM_FAST) return hr::bp_fast_describe(pl->fast, pl->fg, buf, len);
-  if (buf && len > 0)
-    snprintf(buf, (size_t)len, "%s slices_per_thread=%d tile=%dx%d%s", pl->form == HR_FORM_FP64 ? "fp64" : "plain",
-             pl->form == HR_FORM_FP64 ? kNzFp64 : kNzPlain, kBx, kBy,
-             pl->form == HR_FORM_FP64 ? ""
-             : pl->prm.qcap > 0 && plain_q_smem(pl->prm) <= kPlainQSmemMax ? " weights=per-block table"
-                                                                            : " weights=per update");
+  if (buf && len > 0) {
+    const bool fp64 = pl->form == HR_FORM_FP64, table = fp64 ? fp64_q_fits(pl->prm) : plain_q_fits(pl->prm);
+    snprintf(buf, (size_t)len, "%s slices_per_thread=%d tile=%dx%d weights=%s", fp64 ? "fp64" : "plain",
+             !fp64 ? kNzPlain : table ? kNzFp64Q : kNzFp64, !table ? kBx : fp64 ? kDx : kTx,
+             !table ? kBy : fp64 ? kDy : kTy, table ? "per-block table" : "per update");
+  }
   return HR_OK;
 }
 
