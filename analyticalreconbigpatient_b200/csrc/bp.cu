@@ -294,6 +294,23 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// a + f (b - a). WEIGHTED: (1 - f) a + f b, which stays infinite, with its sign, where one of them is (the
+// difference form is then NaN) and does not overflow where both are finite.
+template <bool WEIGHTED>
+__device__ __forceinline__ uint64_t lerp2(uint64_t f, uint64_t a, uint64_t b) {
+  if constexpr (WEIGHTED) return fma2(f, b, mul2(sub2(kOne2, f), a));
+  return fma2(f, sub2(b, a), a);
+}
+template <bool WEIGHTED>
+__device__ __forceinline__ double lerp(double f, double a, double b) {
+  if constexpr (WEIGHTED) return fma(f, b, (1.0 - f) * a);
+  return fma(f, b - a, a);
+}
 
 // Data pointer plus a row's bytes in one wide multiply-add.
 template <class T>
@@ -305,7 +322,7 @@ __device__ __forceinline__ const T* row_ptr(const T* base, uint32_t row, uint32_
 // Four slices of a column, from `first`: their taps, two slices to a packed
 // register pair, weighted and added. TEST: slices whose row is off the detector
 // or whose q2 is negative are left out (else all are known to count).
-template <int NZ, bool TEST>
+template <int NZ, bool TEST, bool WEIGHTED>
 __device__ __forceinline__ void plain_group(float (&res)[NZ], int first, const uint32_t (&row)[4], uint32_t rows,
                                             const float (&fz)[4], const float* c0, const float* c1, uint32_t pitch,
                                             uint64_t ux2, uint64_t E2, float4 q4) {
@@ -324,11 +341,11 @@ __device__ __forceinline__ void plain_group(float (&res)[NZ], int first, const u
 #pragma unroll
   for (int i = 0; i < 4; i += 2) {
     const uint64_t A0 = pk2(a0[i], a0[i + 1]), A1 = pk2(a1[i], a1[i + 1]);
-    const uint64_t ra = fma2(ux2, sub2(pk2(b0[i], b0[i + 1]), A0), A0);
-    const uint64_t rb = fma2(ux2, sub2(pk2(b1[i], b1[i + 1]), A1), A1);
+    const uint64_t ra = lerp2<WEIGHTED>(ux2, A0, pk2(b0[i], b0[i + 1]));
+    const uint64_t rb = lerp2<WEIGHTED>(ux2, A1, pk2(b1[i], b1[i + 1]));
     const uint64_t f2 = add2(pk2(fz[i], fz[i + 1]), kNegOne2);  // [1, 2) -> [0, 1)
     float tap[2], den2[2];
-    up2(fma2(f2, sub2(rb, ra), ra), tap[0], tap[1]);
+    up2(lerp2<WEIGHTED>(f2, ra, rb), tap[0], tap[1]);
     up2(fma2(pk2(q2[i], q2[i + 1]), E2, kOne2), den2[0], den2[1]);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -349,7 +366,7 @@ struct PlainColumn {
 
 // Views [q0, q1) of the block's union window for one column. ALL: every slice
 // of the block has every view of the range in its window (no window tests).
-template <int NZ, bool ALL>
+template <int NZ, bool ALL, bool WEIGHTED = false>
 __device__ __forceinline__ void plain_views(float (&res)[NZ], const PlainColumn& C, const BpParams& P, int q0, int q1) {
   const size_t plane = (size_t)P.ZL * P.YL;
   const uint32_t rows = (uint32_t)(P.ZL - 1), chans = (uint32_t)(P.YL - 1);
@@ -418,11 +435,64 @@ __device__ __forceinline__ void plain_views(float (&res)[NZ], const PlainColumn&
       if (!in0 && !in3 && (int)(row[0] ^ row[3]) >= 0) continue;  // all on one side of the detector
       const bool inside = in0 && in3;
       if (ALL && inside)
-        plain_group<NZ, false>(res, 4 * h, row, rows, fz, c0, c1, pitch, ux2, E2, qrow[h]);
+        plain_group<NZ, false, WEIGHTED>(res, 4 * h, row, rows, fz, c0, c1, pitch, ux2, E2, qrow[h]);
       else
-        plain_group<NZ, true>(res, 4 * h, row, rows, fz, c0, c1, pitch, ux2, E2, qrow[h]);
+        plain_group<NZ, true, WEIGHTED>(res, 4 * h, row, rows, fz, c0, c1, pitch, ux2, E2, qrow[h]);
     }
   }
+}
+
+// Shared memory of a table-weight CTA (T: float or double), and the union view
+// window of its NZ slices.
+template <class T, int NZ>
+struct BlockTables {
+  double* z;         // [NZ] voxel z of the block's slices
+  int *s0, *lo, *hi; // [NZ] central view and clamped window [lo, hi]
+  T* q;              // [qcap][NZ]
+  __device__ __forceinline__ explicit BlockTables(unsigned char* smem)
+      : z(reinterpret_cast<double*>(smem)), s0(reinterpret_cast<int*>(z + NZ)), lo(s0 + NZ), hi(lo + NZ),
+        q(reinterpret_cast<T*>(hi + NZ)) {
+    static_assert(NZ % 2 == 0, "q on a boundary of 8 bytes");
+  }
+  __device__ __forceinline__ int first() const {
+    int p = lo[0];
+    for (int m = 1; m < NZ; ++m) p = min(p, lo[m]);
+    return p;
+  }
+  __device__ __forceinline__ int last() const {
+    int p = hi[0];
+    for (int m = 1; m < NZ; ++m) p = max(p, hi[m]);
+    return p;
+  }
+};
+
+// An infinite sample among the taps of plain_views' differences gives NaN: the
+// thread's NaN voxels again, with weighted taps. (Weighted taps for all would
+// cost 4 to 7 % of the kernel's time; this costs 0.3 %, in FP64 1.4 %, and a
+// volume of nothing but NaN is computed twice.) Neither inlined nor given what
+// it can derive, so that the views' loop keeps its registers.
+template <int NZ>
+__device__ __noinline__ void plain_nan_voxels(float* vol, const float* fp, const ViewTab* views, const BpParams& P,
+                                              unsigned char* smem) {
+  const BlockTables<float, NZ> B(smem);
+  const int xi = blockIdx.x * kTx + threadIdx.x, yi = blockIdx.y * kTy + threadIdx.y, z0 = blockIdx.z * NZ;
+  PlainColumn C;
+  C.fp = fp;
+  C.views = views;
+  C.q_s = B.q;
+  C.z_s = B.z;
+  C.x = __dmul_rn(__dsub_rn((double)xi, P.XNC), P.dx);
+  C.y = __dmul_rn(__dsub_rn((double)yi, P.YNC), P.dy);
+  C.z00 = B.z[0];
+  C.pstart = B.first();
+  float res[NZ];
+#pragma unroll
+  for (int m = 0; m < NZ; ++m) res[m] = 0.0f;
+  plain_views<NZ, false, true>(res, C, P, 0, min(B.last() - C.pstart + 1, P.qcap));
+  float* out = vol + ((size_t)yi * P.XN + xi) * P.ZN + z0;
+#pragma unroll
+  for (int m = 0; m < NZ; ++m)
+    if (z0 + m < P.ZN && isnan(out[m])) out[m] = res[m] * P.DeltaFaif;
 }
 
 template <int NZ>
@@ -431,11 +501,10 @@ __global__ void __launch_bounds__(kTx* kTy, 4) bp_plain_q_kernel(float* __restri
                                                              const float* __restrict__ gw, const __grid_constant__ BpParams P) {
   static_assert(NZ % 4 == 0, "slices are processed in groups of four");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* z_s = reinterpret_cast<double*>(smem_raw);        // [NZ] voxel z of the block's slices
-  int* s0_s = reinterpret_cast<int*>(z_s + NZ);             // [NZ] central view
-  int* lo_s = s0_s + NZ;                                     // [NZ] clamped window [lo, hi]
-  int* hi_s = lo_s + NZ;                                     // [NZ]
-  float* q_s = reinterpret_cast<float*>(hi_s + NZ);          // [qcap][NZ]
+  const BlockTables<float, NZ> B(smem_raw);
+  double* z_s = B.z;
+  int *s0_s = B.s0, *lo_s = B.lo, *hi_s = B.hi;
+  float* q_s = B.q;
   const int tid = threadIdx.y * kTx + threadIdx.x;
   const int z0 = blockIdx.z * NZ;
   // the block's union window (uniform over the CTA; every thread evaluates it)
@@ -500,9 +569,13 @@ __global__ void __launch_bounds__(kTx* kTy, 4) bp_plain_q_kernel(float* __restri
   plain_views<NZ, true>(res, C, P, qa, qb);
   plain_views<NZ, false>(res, C, P, qb, len);
   float* out = vol + ((size_t)yi * P.XN + xi) * P.ZN + z0;
+  bool nan = false;
 #pragma unroll
-  for (int m = 0; m < NZ; ++m)
+  for (int m = 0; m < NZ; ++m) {
     if (z0 + m < P.ZN) out[m] = res[m] * P.DeltaFaif;
+    nan = nan || isnan(res[m]);
+  }
+  if (nan) plain_nan_voxels<NZ>(vol, fp, views, P, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -604,64 +677,11 @@ __device__ __noinline__ double fp64_update_exact(const BpParams& P, const double
 
 constexpr int kDx = 8, kDy = 32;  // CTA tile (x, y)
 
-template <int NZ>
-__global__ void __launch_bounds__(kDx* kDy, 3) bp_fp64_q_kernel(double* __restrict__ vol, const double* __restrict__ fp,
-                                                               const ViewTab* __restrict__ views,
-                                                               const double* __restrict__ gw,
-                                                               const __grid_constant__ BpParams P) {
-  static_assert(NZ % 2 == 0, "slices are processed in pairs");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* z_s = reinterpret_cast<double*>(smem_raw);  // [NZ]
-  int* s0_s = reinterpret_cast<int*>(z_s + NZ);       // [NZ] central view
-  int* lo_s = s0_s + NZ;                              // [NZ] clamped window [lo, hi]
-  int* hi_s = lo_s + NZ;                              // [NZ]
-  double* q_s = reinterpret_cast<double*>(hi_s + NZ + (NZ & 1));  // [qcap][NZ]
-  const int tid = threadIdx.y * kDx + threadIdx.x;
-  const int z0 = blockIdx.z * NZ;
-  int pstart = 0x7fffffff, pend = -0x7fffffff;
-#pragma unroll
-  for (int m = 0; m < NZ; ++m) {
-    const ZInfo zi = z_info(P, z0 + m);
-    if (tid == 0) {
-      z_s[m] = zi.z;
-      s0_s[m] = zi.s0;
-      lo_s[m] = zi.lo;
-      hi_s[m] = zi.hi;
-    }
-    pstart = min(pstart, zi.lo);
-    pend = max(pend, zi.hi);
-  }
-  int len = pend >= pstart ? pend - pstart + 1 : 0;  // 0: every slice lies outside the scan
-  if (len > P.qcap) len = P.qcap;                    // the host sizes qcap from the same expressions
-  __syncthreads();
-  for (int e = tid; e < len * NZ; e += kDx * kDy) {
-    const int q = e / NZ, m = e - q * NZ;
-    const int p = pstart + q;
-    double qv = -1.0;
-    if (p >= lo_s[m] && p <= hi_s[m]) {
-      const int before = p < s0_s[m];
-      const int d1 = (int)(P.N_pi - (double)(s0_s[m] - p));
-      const int d2 = before ? (int)(d1 + P.N_pi) : (int)(d1 - P.N_pi);
-      const double w1 = __ldg(gw + d1), w2 = __ldg(gw + d2);
-      const double t2 = __dsub_rn(z_s[m], views[p].hv);
-      const double tc = before ? t2 - 0.5 : t2 + 0.5;
-      // infinite where w1 or tc is 0 (weight 0: a bound keeps the reciprocal finite), NaN where the
-      // reference's weight is
-      const double r = w2 / w1 * pow(fabs(t2) / fabs(tc), P.k1);
-      qv = r > kBig ? kBig : r;
-    }
-    q_s[e] = qv;
-  }
-  __syncthreads();
-  const int xi = blockIdx.x * kDx + threadIdx.x;
-  const int yi = blockIdx.y * kDy + threadIdx.y;
-  if (xi >= P.XN || yi >= P.YN) return;
-  const double x = __dmul_rn(__dsub_rn((double)xi, P.XNC), P.dx);
-  const double y = __dmul_rn(__dsub_rn((double)yi, P.YNC), P.dy);
-  const double z00 = __dmul_rn(__dsub_rn((double)z0, P.ZNC), P.dz);
-  double res[NZ];
-#pragma unroll
-  for (int m = 0; m < NZ; ++m) res[m] = 0.0;
+// The views of a block's union window for one column.
+template <int NZ, bool WEIGHTED>
+__device__ __forceinline__ void fp64_views(double (&res)[NZ], const double* __restrict__ fp,
+                                           const ViewTab* __restrict__ views, const double* q_s, const double* z_s,
+                                           const BpParams& P, double x, double y, double z00, int pstart, int len) {
   const size_t plane = (size_t)P.ZL * P.YL;
   const uint32_t rows = (uint32_t)(P.ZL - 1), chans = (uint32_t)(P.YL - 1);
   const uint32_t pitch = (uint32_t)P.YL * (uint32_t)sizeof(double);
@@ -735,9 +755,9 @@ __global__ void __launch_bounds__(kDx* kDy, 3) bp_fp64_q_kernel(double* __restri
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const double ra = fma(ux, b0[i] - a0[i], a0[i]);
-        const double rb = fma(ux, b1[i] - a1[i], a1[i]);
-        const double tap = fma(vd[i] + 0.5, rb - ra, ra);
+        const double ra = lerp<WEIGHTED>(ux, a0[i], b0[i]);
+        const double rb = lerp<WEIGHTED>(ux, a1[i], b1[i]);
+        const double tap = lerp<WEIGHTED>(vd[i] + 0.5, ra, rb);
         const double s = fma(q2[i], E, 1.0);
         double w = rcp64_approx(s);
         w = fma(fma(-s, w, 1.0), w, w);
@@ -746,10 +766,93 @@ __global__ void __launch_bounds__(kDx* kDy, 3) bp_fp64_q_kernel(double* __restri
       }
     }
   }
+}
+
+// The thread's NaN voxels with weighted taps, as in the plain form.
+template <int NZ>
+__device__ __noinline__ void fp64_nan_voxels(double* vol, const double* fp, const ViewTab* views, const BpParams& P,
+                                             unsigned char* smem) {
+  const BlockTables<double, NZ> B(smem);
+  const int xi = blockIdx.x * kDx + threadIdx.x, yi = blockIdx.y * kDy + threadIdx.y, z0 = blockIdx.z * NZ;
+  const double x = __dmul_rn(__dsub_rn((double)xi, P.XNC), P.dx);
+  const double y = __dmul_rn(__dsub_rn((double)yi, P.YNC), P.dy);
+  const int pstart = B.first();
+  double res[NZ];
+#pragma unroll
+  for (int m = 0; m < NZ; ++m) res[m] = 0.0;
+  fp64_views<NZ, true>(res, fp, views, B.q, B.z, P, x, y, B.z[0], pstart, min(B.last() - pstart + 1, P.qcap));
   double* out = vol + ((size_t)yi * P.XN + xi) * P.ZN + z0;
 #pragma unroll
   for (int m = 0; m < NZ; ++m)
+    if (z0 + m < P.ZN && isnan(out[m])) out[m] = res[m] * P.DeltaFai;
+}
+
+template <int NZ>
+__global__ void __launch_bounds__(kDx* kDy, 3) bp_fp64_q_kernel(double* __restrict__ vol, const double* __restrict__ fp,
+                                                               const ViewTab* __restrict__ views,
+                                                               const double* __restrict__ gw,
+                                                               const __grid_constant__ BpParams P) {
+  static_assert(NZ % 2 == 0, "slices are processed in pairs");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const BlockTables<double, NZ> B(smem_raw);
+  double* z_s = B.z;
+  int *s0_s = B.s0, *lo_s = B.lo, *hi_s = B.hi;
+  double* q_s = B.q;
+  const int tid = threadIdx.y * kDx + threadIdx.x;
+  const int z0 = blockIdx.z * NZ;
+  int pstart = 0x7fffffff, pend = -0x7fffffff;
+#pragma unroll
+  for (int m = 0; m < NZ; ++m) {
+    const ZInfo zi = z_info(P, z0 + m);
+    if (tid == 0) {
+      z_s[m] = zi.z;
+      s0_s[m] = zi.s0;
+      lo_s[m] = zi.lo;
+      hi_s[m] = zi.hi;
+    }
+    pstart = min(pstart, zi.lo);
+    pend = max(pend, zi.hi);
+  }
+  int len = pend >= pstart ? pend - pstart + 1 : 0;  // 0: every slice lies outside the scan
+  if (len > P.qcap) len = P.qcap;                    // the host sizes qcap from the same expressions
+  __syncthreads();
+  for (int e = tid; e < len * NZ; e += kDx * kDy) {
+    const int q = e / NZ, m = e - q * NZ;
+    const int p = pstart + q;
+    double qv = -1.0;
+    if (p >= lo_s[m] && p <= hi_s[m]) {
+      const int before = p < s0_s[m];
+      const int d1 = (int)(P.N_pi - (double)(s0_s[m] - p));
+      const int d2 = before ? (int)(d1 + P.N_pi) : (int)(d1 - P.N_pi);
+      const double w1 = __ldg(gw + d1), w2 = __ldg(gw + d2);
+      const double t2 = __dsub_rn(z_s[m], views[p].hv);
+      const double tc = before ? t2 - 0.5 : t2 + 0.5;
+      // infinite where w1 or tc is 0 (weight 0: a bound keeps the reciprocal finite), NaN where the
+      // reference's weight is
+      const double r = w2 / w1 * pow(fabs(t2) / fabs(tc), P.k1);
+      qv = r > kBig ? kBig : r;
+    }
+    q_s[e] = qv;
+  }
+  __syncthreads();
+  const int xi = blockIdx.x * kDx + threadIdx.x;
+  const int yi = blockIdx.y * kDy + threadIdx.y;
+  if (xi >= P.XN || yi >= P.YN) return;
+  const double x = __dmul_rn(__dsub_rn((double)xi, P.XNC), P.dx);
+  const double y = __dmul_rn(__dsub_rn((double)yi, P.YNC), P.dy);
+  const double z00 = __dmul_rn(__dsub_rn((double)z0, P.ZNC), P.dz);
+  double res[NZ];
+#pragma unroll
+  for (int m = 0; m < NZ; ++m) res[m] = 0.0;
+  fp64_views<NZ, false>(res, fp, views, q_s, z_s, P, x, y, z00, pstart, len);
+  double* out = vol + ((size_t)yi * P.XN + xi) * P.ZN + z0;
+  bool nan = false;
+#pragma unroll
+  for (int m = 0; m < NZ; ++m) {
     if (z0 + m < P.ZN) out[m] = res[m] * P.DeltaFai;
+    nan = nan || isnan(res[m]);
+  }
+  if (nan) fp64_nan_voxels<NZ>(vol, fp, views, P, smem_raw);
 }
 
 constexpr int kNzPlain = 8;
@@ -831,7 +934,7 @@ bool plain_q_fits(const BpParams& P) { return P.qcap > 0 && plain_q_smem(P) <= k
 // it (thick slices) the per-update kernel runs.
 static_assert(kNzFp64Q <= kNzPlain, "qcap is the longest union window of kNzPlain slices");
 size_t fp64_q_smem(const BpParams& P) {
-  return sizeof(double) * kNzFp64Q + sizeof(int) * (3 * kNzFp64Q + (kNzFp64Q & 1)) +
+  return sizeof(double) * kNzFp64Q + sizeof(int) * 3 * kNzFp64Q +
          sizeof(double) * (size_t)P.qcap * kNzFp64Q;
 }
 constexpr size_t kFp64QSmemMax = 100 * 1024;
