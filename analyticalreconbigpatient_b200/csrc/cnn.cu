@@ -526,8 +526,16 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
 // stage's gradient chunks for db, and every kWgGroup tiles add the finished accumulator (one
 // of two in TMEM) to FP32 registers with rounding to nearest, so that the tensor core's own
 // accumulation, which truncates, runs over 32 steps at most (left to run over a CTA's whole
-// share it shrinks the gradients by 1.1e-5; over four tiles by 4e-7). A warp reads its TMEM
-// lane quarter (row r for 32 input channels) for one gradient row. Every wait is bounded.
+// share it shrinks the gradients by 1.1e-5; over one, two or four tiles it cannot be told
+// from the rounding of the FP32 sums). A warp reads its TMEM
+// lane quarter (row r for 32 input channels) for one gradient row. At the end a CTA adds up what
+// its warps hold of one gradient (two hold each weight's, eight each bias's) in shared memory
+// and adds the sum to the result once: what is left of rounding are those additions, one
+// after another, 2.5e-8 sqrt(CTAs / 3) of the sum (with an addition per warp the weights of 64
+// CTAs' images were off by 1.4e-7 to 1.7e-7, now 1.2e-7, the biases of 148 CTAs' by 4e-7 to
+// 9e-7, now up to 2e-7; half the additions to memory, or an eighth, also take a training step
+// of eight 512 x 512 from 1.91 to 1.75 ms).
+// Every wait is bounded.
 //
 // The CUDA-core kernel this replaced (36 FP32 accumulators per thread, 13 shared-memory
 // reads per 36 FMAs) took 1.40 ms per 32 -> 32 layer of 8 x 512 x 512, 11.0 of the 12.6 ms
@@ -543,7 +551,8 @@ constexpr int kWgStage = (kWgXPlanes + kWgGPlanes) * kWgPlane;
 constexpr int kWgWorkers = 8;                        // warps 0-7: bias sums and flushes
 constexpr int kWgThreads = 32 * (kWgWorkers + 2);
 constexpr int kWgTmemCols = 512;
-constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256;
+constexpr size_t kWgSmem = (size_t)kWgStages * kWgStage + 256 + kWgWorkers * 32 * sizeof(float);
+static_assert(3 * 32 * 3 * 32 * sizeof(float) <= (size_t)kWgStages * kWgStage, "the weights' sums reuse the ring");
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __restrict__ X,
@@ -563,6 +572,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
   uint64_t* mdone = tempty + 2;          // the MMA issuer's last commit
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* bias_s = reinterpret_cast<float*>(wg_smem + kWgStages * kWgStage + 256);  // [kWgWorkers][COUT]
+  float* sum_s = reinterpret_cast<float*>(wg_smem);  // [3 COUT][3 CIN], once the ring is done with
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int Wp = padded_width(W);
   const uint32_t nseg = (uint32_t)(W + kTileM - 1) / kTileM, npair = (uint32_t)(H + 1) / 2;
@@ -606,16 +617,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
   const uint32_t tiles = (uint32_t)B * npair * nseg;                                 // < 2^31, checked at launch
   const int n = (int)((tiles - blockIdx.x + gridDim.x - 1) / gridDim.x);             // this CTA's (grid <= tiles)
 
+  const int q = warp & 3, g = warp >> 2;  // workers: TMEM lane quarter and gradient row this warp flushes
+  const int m = q * 32 + lane;            // row of D
+  const int r = m / CIN, ci = m - r * CIN, dy = r - g;
+  float acc[3][COUT];
+#pragma unroll
+  for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+    for (int c = 0; c < COUT; ++c) acc[dx][c] = 0.0f;
   if (warp < kWgWorkers) {
     // ---- bias sums and flushes -------------------------------------------------------------------
-    const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter and gradient row this warp flushes
-    const int m = q * 32 + lane;            // row of D
-    const int r = m / CIN, ci = m - r * CIN, dy = r - g;
-    float acc[3][COUT];
-#pragma unroll
-    for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-      for (int c = 0; c < COUT; ++c) acc[dx][c] = 0.0f;
     float bacc[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) bacc[k] = 0.0f;
@@ -673,20 +684,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       if (last >= 1 && (n - 1) % kWgGroup == 0) flush(last - 1);
       if (ok) flush(last);
     }
-    if (ok && dy >= 0 && dy < 3) {
 #pragma unroll
-      for (int dx = 0; dx < 3; ++dx)
+    for (int k = 0; k < 8; ++k) {
 #pragma unroll
-        for (int c = 0; c < COUT; ++c)
-          atomicAdd(dW + ((size_t)c * 9 + 3 * dy + dx) * CIN + ci, acc[dx][c]);
-    }
-    if (ok) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-#pragma unroll
-        for (int o = 16; o >= GC; o >>= 1) bacc[k] += __shfl_xor_sync(0xffffffffu, bacc[k], o);
-        if (lane < GC) atomicAdd(db + 8 * lane + k, bacc[k]);
-      }
+      for (int o = 16; o >= GC; o >>= 1) bacc[k] += __shfl_xor_sync(0xffffffffu, bacc[k], o);
+      if (lane < GC) bias_s[warp * COUT + 8 * lane + k] = bacc[k];
     }
   } else if (warp == kWgWorkers) {
     // ---- MMA issuer -----------------------------------------------------------------------------
@@ -747,10 +749,34 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_tc_kernel(const uint4* __
       mbar_drain(&full[i % kWgStages], (uint32_t)(i / kWgStages) & 1, err, kWaitLimit);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  __syncthreads();  // every copy has landed and every MMA has read its operands: the ring's memory is free
   if (warp == kWgWorkers) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kWgTmemCols));
+  }
+  // The CTA's sums (an aborted one has none): the second gradient row's warps hand theirs to the first's.
+  const bool done = !*abort_flag, mine = warp < kWgWorkers && dy >= 0 && dy < 3;
+  if (done && mine && g == 1) {
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int c = 0; c < COUT; ++c) sum_s[(dx * COUT + c) * 3 * CIN + dy * CIN + ci] = acc[dx][c];
+  }
+  __syncthreads();
+  if (done && mine && g == 0) {
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int c = 0; c < COUT; ++c)
+        atomicAdd(dW + ((size_t)c * 9 + 3 * dy + dx) * CIN + ci,
+                  acc[dx][c] + sum_s[(dx * COUT + c) * 3 * CIN + dy * CIN + ci]);
+  }
+  if (done && tid >= 32 * kWgWorkers && tid < 32 * kWgWorkers + COUT) {  // the MMA warp: a channel's bias to a lane
+    const int c = tid - 32 * kWgWorkers;
+    float sum = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWgWorkers; ++w) sum += bias_s[w * COUT + c];
+    atomicAdd(db + c, sum);
   }
 }
 

@@ -81,3 +81,14 @@ def gradient_errors(cuda, B, H, W, seed):
 def test_weight_gradients_of_known_operands(cuda, B, H, W):
     errors = gradient_errors(cuda, B, H, W, H)
     assert all(w < TOL and b < TOL for w, b in errors), errors
+
+
+def test_sums_of_a_cta_are_added_once(cuda):
+    """The last additions, one per CTA and one after another in FP32, each round by 0.3 of half a unit of the sum so
+    far on average: 2.5e-8 sqrt(N / 3) of the whole for N additions. 64 CTAs (32 pairs of rows, two strips) give
+    1.15e-7 for the 9216 weights of a layer together, two additions per CTA 1.63e-7: the limit is 1.4e-7. 148 CTAs
+    give 1.8e-7 for the biases, of which few differ, so the limit is 6e-7, over three times that; with one per warp
+    (eight per CTA) they are expected 5e-7 off and come out beyond it in one of eight layers."""
+    for seed in (1, 2):
+        assert all(w < 1.4e-7 for w, _ in gradient_errors(cuda, 1, 64, 129, seed)[1:7])
+        assert all(b < 6e-7 for _, b in gradient_errors(cuda, 8, 512, 512, seed))
