@@ -262,7 +262,7 @@ __device__ __forceinline__ float plain_update_exact(const BpParams& P, const flo
 // the slice, so the first and last of four tell whether all lie on the detector
 // (no clamps or tests) or all off one side of it (skipped).
 // Measured on two rotations of 888 x 64 -> 512 x 512 x 48 (8.4e9 updates):
-// 28.8 -> 14.4 ms, 44 instructions per update at 75 % issue, L1 hits 92 %.
+// 28.8 -> 14.4 ms, 47 instructions per update at 73 % issue, L1 hits 92 %.
 // 64 registers (4 CTAs of 256 per SM) 15.24 ms for the chain, 80: 15.53, 96:
 // 17.8; CTAs of 128, which tabulate Q2 twice as often, are slower still.
 constexpr uint32_t kFixRound = 256;             // half of the 9 dropped fraction bits
@@ -650,12 +650,15 @@ __global__ void __launch_bounds__(kBx* kBy) bp_fp64_kernel(double* __restrict__ 
 // units bound it (64 lanes per clock and SM). Here the reciprocals and the root
 // start from the approximate instructions and take two Newton steps (1e-16), V
 // of slice m is v(first) + m dv and its floor two adds: 51 FP64 operations per
-// update, 17 of them per update proper. Where a row lies within 1.2e-7 (a
+// update, 17 of them per update proper. Where a row lies within 2.4e-7 (a
 // channel 1e-9) of an integer the update repeats the reference's own operations
 // (fp64_update_exact), so index selection stays exact; elsewhere values differ
-// from it by rounding only.
+// from it by rounding only: against an evaluation in 80 bits, on smooth data,
+// 7.4e-16, 7.5e-16 and 5.7e-16 relative (three geometries), the kernel above
+// 7.7e-16, 7.5e-16 and 5.5e-16; on noise 4.4e-14, 4.3e-14 and 4.0e-14 against
+// 4.8e-14, 4.8e-14 and 4.1e-14.
 // Measured on 888 x 16, 3 rotations -> 186 x 171 x 21 (4.9e8 updates): 13.6 ->
-// 3.05 ms; eight slices per thread halve the per-view work but need 117
+// 3.1 ms (FP64 pipe 45 %, issue 57 %); eight slices per thread halve the per-view work but need 117
 // registers and leave 1.5 waves of CTAs there: 4.17 ms.
 __device__ __noinline__ double fp64_update_exact(const BpParams& P, const double* __restrict__ fp, const ViewTab v,
                                                  int p, double x, double y, double z, double q2) {
@@ -686,7 +689,7 @@ __device__ __forceinline__ void fp64_views(double (&res)[NZ], const double* __re
   const uint32_t rows = (uint32_t)(P.ZL - 1), chans = (uint32_t)(P.YL - 1);
   const uint32_t pitch = (uint32_t)P.YL * (uint32_t)sizeof(double);
   constexpr double kM = 6755399441055744.0;          // 1.5 * 2^52: adding it rounds to an integer
-  constexpr uint32_t kTie = 0x3fdfffffu;             // high word of |x| >= 0.5 - 1.2e-7
+  constexpr uint32_t kTie = 0x3fdfffffu;             // high word of |x| >= 0.5 - 2.4e-7
 #pragma unroll 1
   for (int q = 0; q < len; ++q) {
     const ViewTab v = views[pstart + q];

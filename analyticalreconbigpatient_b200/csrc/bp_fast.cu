@@ -436,20 +436,6 @@ __global__ void tex_absmax_kernel(float* __restrict__ scale, const uint32_t* __r
   if ((threadIdx.x & 31) == 0 && m) atomicMax(reinterpret_cast<unsigned*>(scale + 1), m);
 }
 
-// BF16 pairs [views][ZL][YL] -> the layered arrays, rows [r0, r1) (rows =
-// views x ZL; one CTA row at a time). FP16 (MODE 0): scaled by 2^k with the
-// largest |value| in [2^14, 2^15); scale[0] = 2^-k, which the backprojection
-// folds into its output. Views filled range by range while the fan data is
-// still arriving (a streamed execution) cannot know the largest |value| of the
-// scan: the first range (MODE 1) puts its own largest |value| in [2^10, 2^11)
-// and keeps the factor in scale[2]; later ranges (MODE 2) reuse it, and
-// scale[3] = 1 records that the running largest |value| (scale[1]) no longer
-// fits below FP16's largest finite value, or that the first range was all
-// zeros, so that the caller refills the whole copy with MODE 0. Any power of
-// two that keeps the values in FP16's normal range gives the same samples up
-// to that power.
-constexpr int kStreamHeadroom = 4;  // binades between the first range's largest |value| and MODE 0's range
-//
 // Rows of a multiple of eight (or four) channels that start on 16-byte boundaries
 // go by CTAs of four rows and threads of eight (four) channels: 16
 // bytes in and out per access, many in flight, and no division per texel group
@@ -496,6 +482,19 @@ __device__ __forceinline__ void fill_rows(const unsigned long long* __restrict__
   }
 }
 
+// BF16 pairs [views][ZL][YL] -> the layered arrays, rows [r0, r1) (rows =
+// views x ZL; one CTA row at a time). FP16 (MODE 0): scaled by 2^k with the
+// largest |value| in [2^14, 2^15); scale[0] = 2^-k, which the backprojection
+// folds into its output. Views filled range by range while the fan data is
+// still arriving (a streamed execution) cannot know the largest |value| of the
+// scan: the first range (MODE 1) puts its own largest |value| in [2^10, 2^11)
+// and keeps the factor in scale[2]; later ranges (MODE 2) reuse it, and
+// scale[3] = 1 records that the running largest |value| (scale[1]) no longer
+// fits below FP16's largest finite value, or that the first range was all
+// zeros, so that the caller refills the whole copy with MODE 0. Any power of
+// two that keeps the values in FP16's normal range gives the same samples up
+// to that power.
+constexpr int kStreamHeadroom = 4;  // binades between the first range's largest |value| and MODE 0's range
 template <bool HALF, int MODE>
 __global__ void tex_fill_kernel(float* __restrict__ scale, const unsigned long long* __restrict__ surfs,
                                 const uint32_t* __restrict__ fpb, long long r0, long long r1, int ZL, int YL,

@@ -533,16 +533,16 @@ __global__ void __launch_bounds__(kThreads, kConvCtas) conv_tc_kernel(const __gr
 // and adds the sum to the result once: what is left of rounding are those additions, one
 // after another, 2.5e-8 sqrt(CTAs / 3) of the sum (with an addition per warp the weights of 64
 // CTAs' images were off by 1.4e-7 to 1.7e-7, now 1.2e-7, the biases of 148 CTAs' by 4e-7 to
-// 9e-7, now up to 2e-7; half the additions to memory, or an eighth, also take a training step
+// 9e-7, now below 4e-7; half the additions to memory, or an eighth, also take a training step
 // of eight 512 x 512 from 1.91 to 1.75 ms).
 // Every wait is bounded.
 //
 // The CUDA-core kernel this replaced (36 FP32 accumulators per thread, 13 shared-memory
 // reads per 36 FMAs) took 1.40 ms per 32 -> 32 layer of 8 x 512 x 512, 11.0 of the 12.6 ms
-// of a training step; this one 0.104 ms. Its MMAs would take 0.04 ms; the copies bound it:
+// of a training step; this one 0.084 ms. Its MMAs would take 0.04 ms; the copies bound it:
 // 0.147 ms with NHWC activations (16 bytes at a time), 0.114 by planes with one thread
 // issuing a tile's 24 copies one after another, 0.104 with a lane to each (fewer MMAs,
-// flushes or bias sums change nothing).
+// flushes or bias sums change nothing), 0.084 with one addition per CTA and weight to memory.
 constexpr int kWgStages = 4;
 constexpr int kWgGroup = 4;                          // tiles accumulated in TMEM before a flush
 constexpr int kWgPlane = kHalo * 16;                 // bytes between planes

@@ -915,7 +915,8 @@ def main():
     bp_ms = res["stages_ms"]["backprojection"]
     bytes_per_update = BYTES_PER_UPDATE_BF16 if chosen == _lib.HR_FORM_FAST else BYTES_PER_UPDATE_FP32
     textured = chosen == _lib.HR_FORM_FAST and "texture" in res["kernels"]
-    kname = (("bp_tex_seg_kernel" if "segmented" in res["kernels"] else "bp_tex_kernel") if textured
+    segmented = "bp_tex_seg_occ_kernel" if any(k in res["kernels"] for k in ("6ctas", "8ctas")) else "bp_tex_seg_kernel"
+    kname = ((segmented if "segmented" in res["kernels"] else "bp_tex_kernel") if textured
              else "bp_fast_kernel") if chosen == _lib.HR_FORM_FAST else "bp_plain_q_kernel"
     achieved = bytes_per_update * updates / (bp_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": pk["hbm_gbs"],
@@ -938,7 +939,8 @@ def main():
                                "frac": samples * 1e9 / rate if rate > 0 else None,
                                "peak_source": "measured (libhelixprobe.so hr_texture_sample_rate: cache-resident FP16 layered "
                                               "texture, every lane active)"}
-        roofline["note"] = ("gather-equivalent bytes (4 FP16 taps = 8 B per update) / backprojection time "
+        roofline["note"] = ("gather-equivalent bytes (4 FP16 taps = 8 B per update, most of which the texture cache "
+                            "serves: the fraction may exceed 1) / backprojection time "
                             "(texture fill included); the taps are bilinear texture samples, so the bound is the "
                             "texture units' sample rate (roofline.texture), not HBM")
 
