@@ -468,7 +468,7 @@ struct BlockTables {
 
 // An infinite sample among the taps of plain_views' differences gives NaN: the
 // thread's NaN voxels again, with weighted taps. (Weighted taps for all would
-// cost 4 to 7 % of the kernel's time; this costs 0.3 %, in FP64 1.4 %, and a
+// cost 4 to 7 % of the kernel's time; this costs 0.3 %, in FP64 1.6 %, and a
 // volume of nothing but NaN is computed twice.) Neither inlined nor given what
 // it can derive, so that the views' loop keeps its registers.
 template <int NZ>
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kBx* kBy) bp_fp64_kernel(double* __restrict__ 
 // 7.4e-16, 7.5e-16 and 5.7e-16 relative (three geometries), the kernel above
 // 7.7e-16, 7.5e-16 and 5.5e-16; on noise 4.4e-14, 4.3e-14 and 4.0e-14 against
 // 4.8e-14, 4.8e-14 and 4.1e-14.
-// Measured on 888 x 16, 3 rotations -> 186 x 171 x 21 (4.9e8 updates): 13.6 ->
+// Measured on 888 x 16, 3 rotations -> 186 x 171 x 21 (4.5e8 updates): 13.6 ->
 // 3.1 ms (FP64 pipe 45 %, issue 57 %); eight slices per thread halve the per-view work but need 117
 // registers and leave 1.5 waves of CTAs there: 4.17 ms.
 __device__ __noinline__ double fp64_update_exact(const BpParams& P, const double* __restrict__ fp, const ViewTab v,
