@@ -116,6 +116,13 @@ def peaks():
     return dict(PEAKS_FALLBACK), "fallback"
 
 
+def texture_kernel(describe: str) -> str:
+    """The texture backprojection kernel that a plan's description names."""
+    if "segmented" not in describe:
+        return "bp_tex_kernel"
+    return "bp_tex_seg_occ_kernel" if "6ctas" in describe or "8ctas" in describe else "bp_tex_seg_kernel"
+
+
 def traffic_from_profiles(kernel: str, config: str):
     """DRAM bytes per launch recorded from an ncu capture (profiles/<kernel>_<config>.md,
     line 'dram_bytes_per_launch: N'), or None."""
@@ -523,8 +530,7 @@ def run_bigpatient(args, scan, dev, world, rank, barrier, emit=True):
     if bp_ms_per_slice:
         upd_per_slice = updates / scan.ZN
         ach = BYTES_PER_UPDATE_BF16 * upd_per_slice / (bp_ms_per_slice * 1e-3) / 1e9
-        roof = {"bound": "hbm", "kernel": ("bp_tex_seg_kernel" if "segmented" in desc else "bp_tex_kernel")
-                if "texture" in desc else "bp_fast_kernel",
+        roof = {"bound": "hbm", "kernel": texture_kernel(desc) if "texture" in desc else "bp_fast_kernel",
                 "achieved": ach, "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": ach / pk["hbm_gbs"], "peak_source": pk_kind, "traffic": None,
                 "note": "gather-equivalent (8 B/update) over the autotuner's best time per slice"}
@@ -915,9 +921,8 @@ def main():
     bp_ms = res["stages_ms"]["backprojection"]
     bytes_per_update = BYTES_PER_UPDATE_BF16 if chosen == _lib.HR_FORM_FAST else BYTES_PER_UPDATE_FP32
     textured = chosen == _lib.HR_FORM_FAST and "texture" in res["kernels"]
-    segmented = "bp_tex_seg_occ_kernel" if any(k in res["kernels"] for k in ("6ctas", "8ctas")) else "bp_tex_seg_kernel"
-    kname = ((segmented if "segmented" in res["kernels"] else "bp_tex_kernel") if textured
-             else "bp_fast_kernel") if chosen == _lib.HR_FORM_FAST else "bp_plain_q_kernel"
+    kname = ((texture_kernel(res["kernels"]) if textured else "bp_fast_kernel")
+             if chosen == _lib.HR_FORM_FAST else "bp_plain_q_kernel")
     achieved = bytes_per_update * updates / (bp_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": pk["hbm_gbs"],
                 "unit": "GB/s", "frac": achieved / pk["hbm_gbs"], "peak_source": pk_kind,
